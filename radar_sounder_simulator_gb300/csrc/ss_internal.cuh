@@ -61,6 +61,20 @@ __device__ __forceinline__ double sinc_np(double y) {
   return sinpi(y) / (kPi * y);
 }
 
+// sinc_np(y1) sinc_np(y2) with one quotient.
+__device__ __forceinline__ double sinc2_np(double y1, double y2) {
+  double num = 1.0, den = 1.0;
+  if (y1 != 0.0) {
+    num = sinpi(y1);
+    den = kPi * y1;
+  }
+  if (y2 != 0.0) {
+    num *= sinpi(y2);
+    den *= kPi * y2;
+  }
+  return num / den;
+}
+
 // Forward-hemisphere cos^(q/2) element field (antenna.py:138-143).
 __device__ __forceinline__ double element_field64(double cb, double q,
                                                   double enabled) {

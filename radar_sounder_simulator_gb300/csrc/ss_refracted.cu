@@ -65,6 +65,7 @@ refracted_fp64_kernel(RefArgs a) {
 
   const int nj = a.leg_last;  // final medium (multilayer.py:506)
   const double n0 = a.n_leg[0], njn = a.n_leg[nj];
+  const double kj = a.k0 * njn, kj_pi = kj / kPi, amp_pref = kj / kTwoPi;
   for (int i = s_rng[0] + tid; i < s_rng[1]; i += blockDim.x) {
     const double q[3] = {(double)a.F.cx[i], (double)a.F.cy[i],
                          (double)a.F.cz[i]};
@@ -80,19 +81,21 @@ refracted_fp64_kernel(RefArgs a) {
         path_joint64<NI == 0 ? 1 : NI>(a, s_p[tt], q, P);
       // final leg (medium j): crossing -> facet
       double d[3] = {P.cur[0] - q[0], P.cur[1] - q[1], P.cur[2] - q[2]};
-      const double s_j = sqrt(dot3v(d, d));
-      const double inv = 1.0 / fmax(s_j, 1e-30);
+      double s_j, inv;
+      sqrt_inv64(fmax(dot3v(d, d), 1e-60), s_j, inv);
       const double rh[3] = {d[0] * inv, d[1] * inv, d[2] * inv};
       const double opl = P.opl + njn * s_j;
-      const double loss = P.loss_db + s_j * (a.att_leg[nj] / 1000.0);
-      const double sperp = P.sum_perp + s_j / njn;
-      const double spar = P.sum_par + s_j / (njn * P.c_last * P.c_last);
-      const double l_perp = n0 * sperp;
-      const double l_par = n0 * P.c0 * P.c0 * spar;
-      const double flux = (n0 * P.c0) / (njn * P.c_last);
-      const double att_f = pow(10.0, -loss / 10.0);
+      const double loss = P.loss_db + s_j * a.att_m[nj];
+      const double sn_j = s_j * a.inv_n[nj];
+      const double sperp = P.sum_perp + sn_j;
+      // spread = tau2 flux / (l_par l_perp), flux = n0 c0 / (nj c_last),
+      // l_par = n0 c0^2 sum_par, l_perp = n0 sum_perp, as one quotient
+      const double cl2 = P.c_last * P.c_last;
+      const double spar_cl2 = P.sum_par * cl2 + sn_j;  // sum_par c_last^2
+      const double att_f = exp10(loss * -0.1);
       const double cos_t = dot3v(rh, fn);
-      double spread = P.tau2 * flux / (l_par * l_perp);
+      double spread = P.tau2 * P.c_last /
+                      (njn * n0 * P.c0 * spar_cl2 * sperp);
       if (a.pat_kind != SS_PAT_ISOTROPIC) {
         double d0[3] = {P.xf[0] - s_p[tt][0], P.xf[1] - s_p[tt][1],
                         P.xf[2] - s_p[tt][2]};
@@ -104,15 +107,13 @@ refracted_fp64_kernel(RefArgs a) {
       double re, im, pwr;
       if (a.coherent) {
         const double gam = a.F.gamma_f64 ? a.F.gamma_f64[i] : a.gamma;
-        const double kj = a.k0 * njn;
         const double f1[3] = {(double)a.F.e1x[i], (double)a.F.e1y[i],
                               (double)a.F.e1z[i]};
         const double f2[3] = {(double)a.F.e2x[i], (double)a.F.e2y[i],
                               (double)a.F.e2z[i]};
         const double d1 = dot3v(rh, f1), d2 = dot3v(rh, f2);
-        const double s1 = sinc_np(d1 * (kj / kPi));
-        const double s2 = sinc_np(d2 * (kj / kPi));
-        double amp = (kj / kTwoPi) * gam * cos_t * fa * s1 * s2 * spread * att_f;
+        double amp = amp_pref * gam * cos_t * fa *
+                     sinc2_np(d1 * kj_pi, d2 * kj_pi) * spread * att_f;
         if (a.taper) {
           double ct = fmin(fmax(cos_t, kCMin), 1.0);
           const double ct2 = ct * ct;
@@ -130,7 +131,7 @@ refracted_fp64_kernel(RefArgs a) {
           const double sk = sg * kk;
           cr = amp * exp(-0.5 * (sk * sk));
           if (fa > 0.0) {
-            const double ai = (kj / kTwoPi) * gam * cos_t * spread * att_f *
+            const double ai = amp_pref * gam * cos_t * spread * att_f *
                               sqrt(dp);
             cr += ai * (double)a.F.phasor[2 * i];
             ci += ai * (double)a.F.phasor[2 * i + 1];
@@ -185,50 +186,65 @@ refracted_fp64_kernel(RefArgs a) {
 // ---------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------
+// Chunk count whose item total (chunks x groups) fills k_min..k_max whole
+// waves of `slots` resident CTAs best (a last wave half full costs a full
+// one); the fewest waves on a tie.
+static int wave_chunks(long slots, int groups, int max_chunks, int k_min,
+                       int k_max) {
+  int best = 1;
+  double best_eff = -1.0;
+  for (int k = k_min; k <= k_max; ++k) {
+    const int nc = (int)std::max<long>(
+        1, std::min<long>(max_chunks, k * slots / groups));
+    const long items = (long)nc * groups;
+    const long waves = (items + slots - 1) / slots;
+    const double eff = (double)items / (double)(waves * slots);
+    if (eff > best_eff + 1e-9) {
+      best_eff = eff;
+      best = nc;
+    }
+  }
+  return best;
+}
+
 static int refracted_plan(const ss_refracted_opts *o, int T, int N, Plan *p) {
   if (o->n_samples <= 0 || T <= 0 || N <= 0 || o->block_size <= 0 ||
       o->n_win <= 0 || o->n_crossed < 1 || o->n_crossed > SS_MAX_IFACE)
     return SS_ERR_ARG;
   const int n_seg = o->n_samples * (o->split_sides ? 2 : 1);
-  const size_t elt = o->precision == SS_PREC_FP64 ? 16 : 8;
+  const bool fp64 = o->precision == SS_PREC_FP64;
+  const size_t elt = fp64 ? 16 : 8;
   const size_t per_trace = (size_t)n_seg * elt;
   if (per_trace > 200 * 1024) return SS_ERR_UNSUPPORTED;
   const size_t budget = 96 * 1024;
   int tb = (int)std::max<size_t>(1, std::min<size_t>(budget / per_trace,
                                                      SS_MAX_TB));
   tb = std::min(tb, T);
-  p->tb = tb;
-  p->n_groups = (T + tb - 1) / tb;
-  p->threads = o->precision == SS_PREC_FP64 ? 128 : kSplitThreads;
+  p->threads = fp64 ? 128 : kSplitThreads;
   const long window = std::min<long>((long)o->n_win * o->block_size, N);
-  const int max_chunks = (int)std::max<long>(1, window / 256);
-  if (o->precision == SS_PREC_FP64) {
-    const int target = 8 * sm_count();
-    p->n_chunks = std::max(
-        1, std::min(max_chunks, (target + p->n_groups - 1) / p->n_groups));
+  if (fp64) {
+    // two resident CTAs per SM at the full histogram budget, three (their
+    // registers) below it. A small call takes smaller trace blocks until
+    // its items cover the SMs: a CTA's work is hundreds of microseconds of
+    // float64 chains, an idle SM cannot be made up for.
+    const int max_chunks = (int)std::max<long>(1, window / 128);
+    const long sms = sm_count();
+    while (tb > 1 && (long)((T + tb - 1) / tb) * max_chunks < 2 * sms)
+      tb = (tb + 1) / 2;
+    const long slots = sms * (tb * per_trace > 72 * 1024 ? 2 : 3);
+    p->n_groups = (T + tb - 1) / tb;
+    p->n_chunks = wave_chunks(slots, p->n_groups, max_chunks, 1, 4);
   } else {
     // resident CTAs per SM of the split kernel that runs: two 512-thread
     // CTAs (64 registers) for the sequential chain and joint solves through
-    // up to two interfaces, one (~128 registers) through three or more; the
-    // chunk count whose item total fills 4-12 whole waves best (a last
-    // wave half full costs a full one), the fewest waves on a tie
+    // up to two interfaces, one (~128 registers) through three or more
+    const int max_chunks = (int)std::max<long>(1, window / 256);
     const long slots = (long)sm_count() *
                        (!o->joint || o->n_crossed <= 2 ? 2 : 1);
-    int best = 1;
-    double best_eff = -1.0;
-    for (int k = 4; k <= 12; ++k) {
-      const int nc = (int)std::max<long>(
-          1, std::min<long>(max_chunks, k * slots / p->n_groups));
-      const long items = (long)nc * p->n_groups;
-      const long waves = (items + slots - 1) / slots;
-      const double eff = (double)items / (double)(waves * slots);
-      if (eff > best_eff + 1e-9) {
-        best_eff = eff;
-        best = nc;
-      }
-    }
-    p->n_chunks = best;
+    p->n_groups = (T + tb - 1) / tb;
+    p->n_chunks = wave_chunks(slots, p->n_groups, max_chunks, 4, 12);
   }
+  p->tb = tb;
   p->smem = (size_t)tb * per_trace;
   return SS_OK;
 }
@@ -342,7 +358,12 @@ int build_ref_args(const ss_refracted_opts *opts,
     a.n_leg[i] = opts->n_leg[i];
     a.eps_leg[i] = opts->eps_leg[i];
     a.att_leg[i] = opts->att_leg[i];
+    a.inv_n[i] = 1.0 / a.n_leg[i];
+    a.att_m[i] = a.att_leg[i] / 1000.0;
+    a.eps_root[i] = sqrt(a.eps_leg[i]);
   }
+  for (int i = 0; i + 1 < n_legs; ++i)
+    a.eps_quot[i] = a.eps_leg[i] / a.eps_leg[i + 1];
   a.rough_cross = opts->sigma_crossed != nullptr;
   a.k0 = opts->k0;
   a.gamma = opts->gamma;

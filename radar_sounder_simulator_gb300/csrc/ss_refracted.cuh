@@ -15,6 +15,10 @@ struct RefArgs {
   ss_interface ifc[SS_MAX_IFACE];
   double n_leg[SS_MAX_IFACE + 1], eps_leg[SS_MAX_IFACE + 1],
       att_leg[SS_MAX_IFACE + 1], sig_c[SS_MAX_IFACE];
+  // per-leg quotients and roots the float64 path would otherwise form per
+  // pair: 1/n, attenuation per metre, sqrt(eps), eps_i / eps_(i+1)
+  double inv_n[SS_MAX_IFACE + 1], att_m[SS_MAX_IFACE + 1],
+      eps_root[SS_MAX_IFACE + 1], eps_quot[SS_MAX_IFACE + 1];
   int rough_cross;
   double k0, gamma, t0, dt, c, taper_s, n_exp;
   int n_samples, n_seg, bs, n_win, split, coherent, joint, n_newton,

@@ -228,14 +228,12 @@ __device__ __forceinline__ bool cell_of(const MeanPlane32 &M,
 }
 
 // Exact reference cell from a float64 mean-plane solve (multilayer.py
-// :375-381 for comp = true, refraction_joint sequential chain for false).
+// :375-381, and the joint path's chain).
 static __device__ __noinline__ void cell64(const ss_interface &I, const double *cur,
                                     const double *q, double n1, double n2,
-                                    bool comp, double *x_out, int &row,
-                                    int &col) {
+                                    double *x_out, int &row, int &col) {
   Snell64 R;
-  snell64(cur, q, I.mean_point, I.mean_normal, n1, n2, 10, comp, R, true,
-          true);
+  snell64(cur, q, I.mean_point, I.mean_normal, n1, n2, 10, R, true);
   const double rc0 = __dadd_rn(__dadd_rn(__dmul_rn(R.x[0], I.coef[0]),
                                          __dmul_rn(R.x[1], I.coef[2])),
                                I.coef[4]);
@@ -469,8 +467,7 @@ __device__ __forceinline__ void path_sequential_split(const RefArgs &a,
         double cur64[3], q64[3] = {q[0], q[1], q[2]}, x1[3];
         for (int j = 0; j < 3; ++j)
           cur64[j] = i == 0 ? p64[j] : (double)o_prev[j] + (double)y_prev[j];
-        cell64(I, cur64, q64, a.n_leg[i], a.n_leg[i + 1], true, x1, row,
-               col);
+        cell64(I, cur64, q64, a.n_leg[i], a.n_leg[i + 1], x1, row, col);
       }
     }
     float o[3], n[3], tn[3];
@@ -599,7 +596,7 @@ __device__ __forceinline__ void path_joint_split(const RefArgs &a, const RefSpli
         double c64[3] = {p64[0], p64[1], p64[2]};
         const double q64[3] = {q[0], q[1], q[2]};
         for (int i = 0; i < ni; ++i)
-          cell64(a.ifc[i], c64, q64, a.n_leg[i], a.n_leg[i + 1], false, c64,
+          cell64(a.ifc[i], c64, q64, a.n_leg[i], a.n_leg[i + 1], c64,
                  rows[i], cols[i]);
       }
     }
