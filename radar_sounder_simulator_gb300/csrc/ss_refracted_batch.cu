@@ -71,6 +71,10 @@ struct RefBatchLayout {
   int path_class = 0, rough_kind = 0, plain = 1;
 };
 
+// Path class of a batch whose sequential jobs all cross one interface
+// (kOneNI kernels); 0 is the general sequential chain, 1-4 the joint solve.
+constexpr int kBatchOne = 5;
+
 static bool job_plain(const RefArgs &a) {
   return a.rough_kind == SS_ROUGH_NONE && a.pat_kind == SS_PAT_ISOTROPIC &&
          !a.taper && !a.F.diffuse_amp && !a.split;
@@ -98,6 +102,7 @@ static int ref_batch_layout(const ss_refracted_job *jobs, int n_jobs,
   }
   L.jobs.assign(n_jobs, RefBatchJob{});
   double total_pairs = 0.0;
+  bool all_one = true;
   std::vector<long long> window(n_jobs);
   for (int j = 0; j < n_jobs; ++j) {
     const ss_refracted_job &q = jobs[j];
@@ -131,6 +136,7 @@ static int ref_batch_layout(const ss_refracted_job *jobs, int n_jobs,
       return SS_ERR_ARG;
     }
     L.plain = L.plain && job_plain(a);
+    all_one = all_one && one_crossing(a);
     const size_t per_trace = (size_t)a.n_seg * sizeof(float2);
     a.tb = (int)std::min<size_t>(
         std::max<size_t>(1, std::min<size_t>(96 * 1024 / per_trace, max_tb)),
@@ -139,6 +145,7 @@ static int ref_batch_layout(const ss_refracted_job *jobs, int n_jobs,
     window[j] = std::min<long long>((long long)a.n_win * a.bs, a.N);
     total_pairs += (double)a.T * window[j];
   }
+  if (all_one) L.path_class = kBatchOne;
   const double per_item =
       std::max(1.0, total_pairs / ((double)ips * sm_count()));
   // The queue serves the costliest jobs first (longest-processing-time
@@ -212,6 +219,7 @@ static int ref_batch_occupancy_class(int cls, int rough, bool plain,
     case 1: return refracted_batch_occupancy_ni1(rough, plain, smem);
     case 2: return refracted_batch_occupancy_ni2(rough, plain, smem);
     case 3: return refracted_batch_occupancy_ni3(rough, plain, smem);
+    case kBatchOne: return refracted_batch_occupancy_nione(rough, plain, smem);
     default: return refracted_batch_occupancy_ni4(rough, plain, smem);
   }
 }
@@ -309,6 +317,7 @@ extern "C" int ss_refracted_batch_run(const ss_refracted_batch_info *info,
     case 1: s = SS_RB(1); break;
     case 2: s = SS_RB(2); break;
     case 3: s = SS_RB(3); break;
+    case kBatchOne: s = SS_RB(one); break;
     default: s = SS_RB(4); break;
   }
 #undef SS_RB

@@ -3,6 +3,8 @@
 // precision design are described in ss_refracted_split.cuh; each
 // interface count is compiled in its own translation unit
 // (ss_refracted_split_ni*.cu) so the build runs them in parallel.
+#include <cmath>
+
 #include "ss_refracted_split.cuh"
 
 namespace ss {
@@ -34,6 +36,44 @@ RefSplitConsts split_consts(const RefArgs &a) {
   // single crossings agree with the float64 path to ~1e-9 m.
   const double og = (!a.joint && a.ni > 1) ? kOplGuardChain : 0.0;
   k.bin_guard = (float)std::max((double)kBinGuard, og * 2.0 / (a.c * a.dt));
+  k.gamma = (float)a.gamma;
+  {
+    OnePlane &O = k.one;
+    const ss_interface &I = a.ifc[0];
+    double mn[3];
+    for (int j = 0; j < 3; ++j) {
+      mn[j] = I.mean_normal[j];
+      O.mp[j] = (float)I.mean_point[j];
+      O.mn[j] = (float)mn[j];
+    }
+    for (int c = 0; c < 4; ++c) {
+      const df cd = df_from_double(I.coef[c]);
+      O.c[c] = cd.hi;
+      O.cl[c] = cd.lo;
+    }
+    for (int c = 0; c < 2; ++c) {
+      const df cd = df_from_double(I.coef[4 + c]);
+      O.c4[c] = cd.hi;
+      O.c4l[c] = cd.lo;
+      O.cn[c] = (float)(I.coef[c] * mn[0] + I.coef[2 + c] * mn[1]);
+    }
+    const double n1 = a.n_leg[0], n2 = a.n_leg[1];
+    O.up = n1 <= n2;
+    O.r = (float)(std::min(n1, n2) / std::max(n1, n2));
+    O.vec = (reinterpret_cast<uintptr_t>(I.table) & 7) == 0;
+    OneLegs &l = k.legs;
+    const df d1 = df_from_double(n1), d2 = df_from_double(n2);
+    l.n1 = d1.hi;
+    l.n1l = d1.lo;
+    l.n2 = d2.hi;
+    l.n2l = d2.lo;
+    l.i1 = (float)(1.0 / n1);
+    l.i2 = (float)(1.0 / n2);
+    // 10^(-loss / 10) = 2^(x1 s1 + x2 s2)
+    const double x = -std::log2(10.0) / 10.0 / 1000.0;
+    l.x1 = (float)(x * a.att_leg[0]);
+    l.x2 = (float)(x * a.att_leg[1]);
+  }
   for (int i = 0; i <= a.leg_last; ++i) {
     const df n = df_from_double(a.n_leg[i]);
     k.n_leg[i] = n.hi;
@@ -67,6 +107,16 @@ RefSplitConsts split_consts(const RefArgs &a) {
   return k;
 }
 
+bool one_crossing(const RefArgs &a) {
+  if (a.joint || a.ni != 1 || a.leg_last != 1) return false;
+  for (int i = 0; i < 2; ++i)
+    if (!(std::fabs(a.n_leg[i] * a.n_leg[i] - a.eps_leg[i]) <=
+          1e-9 * a.eps_leg[i]))
+      return false;
+  // cell indices are clamped as exact float32 integers
+  return a.ifc[0].ny < (1 << 22) && a.ifc[0].nx < (1 << 22);
+}
+
 // Dynamic shared memory of the fast kernel: the trace block's histograms
 // and the series table.
 size_t split_smem_bytes(const RefArgs &a, int tb) {
@@ -83,6 +133,7 @@ int refracted_split_launch(RefArgs &a, const Plan &p, cudaStream_t st) {
   }
   const RefSplitConsts k = split_consts(a);
   const size_t smem = split_smem_bytes(a, p.tb);
+  if (one_crossing(a)) return split_launch_one(a, k, p, smem, st);
   if (!a.joint) return split_launch_ni0(a, k, p, smem, st);
   switch (a.ni) {
     case 1: return split_launch_ni1(a, k, p, smem, st);

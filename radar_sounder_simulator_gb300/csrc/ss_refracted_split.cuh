@@ -48,6 +48,7 @@
 #include "ss_df.cuh"
 #include "ss_f32.cuh"
 #include "ss_refracted_fp64.cuh"
+#include "ss_refracted_one.cuh"
 
 namespace ss {
 
@@ -62,6 +63,10 @@ constexpr float kLookupGuard = 1.5e-4f;
 // (~6x their largest float32 optical-path error, 8.6e-6 m).
 constexpr float kBinGuard = 1e-6f;
 constexpr double kOplGuardChain = 5e-5;
+// Path-class argument of the kernels: 0 the sequential chain, 1-4 and
+// kDeepNI the joint solve through that many interfaces, kOneNI the
+// sequential solve of a single crossing (ss_refracted_one.cuh).
+constexpr int kOneNI = -1;
 
 // Per-interface constants of the float32 lookup pass.
 struct MeanPlane32 {
@@ -75,7 +80,7 @@ struct MeanPlane32 {
 };
 
 struct RefSplitConsts {
-  float k0, amp_pref_j, kj, taper_inv, sigma, corr, fadL, n_exp;
+  float k0, amp_pref_j, kj, taper_inv, sigma, corr, fadL, n_exp, gamma;
   float K2h, K2l;             // 2 k0 as double-float
   float Ah, Al, Bh, Bl;       // u = opl A - B, A = 2/(c dt), B = t0/dt
   float bin_guard;            // bin-edge band in bins (kBinGuard, kOplGuardChain)
@@ -86,6 +91,8 @@ struct RefSplitConsts {
   // rate is the differentiated parameter
   float att_mask[SS_MAX_IFACE + 1];
   MeanPlane32 mean[SS_MAX_IFACE];
+  OnePlane one;   // single-crossing path (kOneNI)
+  OneLegs legs;
 };
 
 __device__ __forceinline__ float dot3a(const float *a, const float *b) {
@@ -904,6 +911,12 @@ __device__ __forceinline__ void load_trace(const RefArgs &a, int t, TraceS &T,
     pv[j] = (a.pv && j < a.pv_len) ? (float)a.pv[a.pv_len * t + j] : 0.0f;
 }
 
+// The same position for the single-crossing path: (hi, lo.x), (lo.y, lo.z).
+__device__ __forceinline__ void stage_trace4(const TraceS &T, float4 *t4) {
+  t4[0] = make_float4(T.ph[0], T.ph[1], T.ph[2], T.pl[0]);
+  t4[1] = make_float4(T.pl[1], T.pl[2], 0.0f, 0.0f);
+}
+
 // Result of one (trace, facet) pair.
 struct PairOut {
   float re, im, pwr;
@@ -925,64 +938,73 @@ struct PairGrad {
   float dloss;
 };
 
-template <int NI, int ROUGH, bool EXACT, bool GRAD = false,
-          bool PLAIN = false>
-__device__ __forceinline__ bool pair_eval(
-    const RefArgs &a, const RefSplitConsts &k, const TraceS &T,
-    const double *p64, const float *u, const float *pv, const float *pat,
-    int pa_len, const float *lg, const float *fad, int i, const float *q,
-    PairOut &o, PairGrad *pg = nullptr) {
-  PathS P;
-  if (NI == 0)
-    path_sequential_split<EXACT, GRAD>(a, k, T, p64, q, P);
-  else
-    path_joint_split<NI == 0 ? 1 : NI, EXACT, GRAD>(a, k, T, p64, q, P);
-  if (!EXACT && P.defer) return false;
-  const int nj = a.leg_last;
-  const float n0 = k.n_leg[0], njn = k.n_leg[nj];
-  const float nsf = (float)a.n_samples;
-  const float fn[3] = {a.F.nx[i], a.F.ny[i], a.F.nz[i]};
-  const float fa = a.F.area[i];
-  // final leg (medium j)
-  const df opl = df_add(P.opl, df_mul(P.s_last, df_make(k.n_leg[nj],
-                                                        k.n_leg_lo[nj])));
-  const float s_j = P.s_last.hi;
-  const float *rh = P.rh;
-  const float loss = P.loss_db + s_j * (k.att_leg[nj] * 1e-3f);
-  const float sperp = P.sum_perp + s_j / njn;
-  const float spar = P.sum_par + s_j / (njn * P.c_last * P.c_last);
-  const float l_perp = n0 * sperp;
-  const float l_par = n0 * P.c0 * P.c0 * spar;
-  const float flux = (n0 * P.c0) / (njn * P.c_last);
-  const float att_f = exp2f(-loss * 0.33219280949f);  // 10^(-loss/10)
-  const float cos_t = dot3a(rh, fn);
-  float spread = P.tau2 * flux / (l_par * l_perp);
+// Facet record of one pair: geometry and, for rough targets, the series'
+// parameters.
+struct FacetS {
+  float q[3], n[3], e1[3], e2[3], area, gam;
+  float sg, lc, l1, l2, phr, phi;  // ROUGH only
+};
+
+template <int ROUGH>
+__device__ __forceinline__ void load_facet(const RefArgs &a,
+                                           const RefSplitConsts &k, int i,
+                                           FacetS &f) {
+  f.n[0] = a.F.nx[i]; f.n[1] = a.F.ny[i]; f.n[2] = a.F.nz[i];
+  f.area = a.F.area[i];
+  if (!a.coherent) return;
+  f.e1[0] = a.F.e1x[i]; f.e1[1] = a.F.e1y[i]; f.e1[2] = a.F.e1z[i];
+  f.e2[0] = a.F.e2x[i]; f.e2[1] = a.F.e2y[i]; f.e2[2] = a.F.e2z[i];
+  f.gam = a.F.gamma_f64 ? (float)a.F.gamma_f64[i] : k.gamma;
+  if (ROUGH != SS_ROUGH_NONE) {
+    f.sg = a.F.sigma ? a.F.sigma[i] : k.sigma;
+    f.lc = a.F.corr ? a.F.corr[i] : k.corr;
+    f.l1 = sqrtf(dot3a(f.e1, f.e1));
+    f.l2 = sqrtf(dot3a(f.e2, f.e2));
+    f.phr = a.F.phasor[2 * i];
+    f.phi = a.F.phasor[2 * i + 1];
+  }
+}
+
+// Contribution and bin of a pair whose path is solved (multilayer.py
+// :500-583): facet response at the local wavenumber, roughness, diffuse
+// channel, carrier phase and fast-time bin. `v`: facet minus platform
+// (side split). `exact_bin(fb)` decides the bin of a pair near a bin edge,
+// or returns false to defer it.
+template <int ROUGH, bool GRAD, bool PLAIN, class ExactBin>
+__device__ __forceinline__ bool pair_finish(
+    const RefArgs &a, const RefSplitConsts &k, const FacetS &f,
+    const PairGeo &G, const float *v, const float *u, const float *pv,
+    const float *pat, int pa_len, const float *lg, const float *fad, int i,
+    PairOut &o, PairGrad *pg, ExactBin exact_bin) {
+  const float *rh = G.rh;
+  const float fa = f.area;
+  const float cos_t = dot3a(rh, f.n);
+  float spread = G.spread;
   if (!PLAIN && a.pat_kind != SS_PAT_ISOTROPIC) {
-    const float dm = rsqrtf(fmaxf(dot3a(P.d0, P.d0), 1e-30f));
+    const float dm = rsqrtf(fmaxf(dot3a(G.d0, G.d0), 1e-30f));
     const float g = gain32(a.pat_kind, a.pat_n, pa_len, pat, pv,
-                           P.d0[0] * dm, P.d0[1] * dm, P.d0[2] * dm);
+                           G.d0[0] * dm, G.d0[1] * dm, G.d0[2] * dm);
     spread *= g * g;
   }
   float re, im, pwr;
   if (a.coherent) {
-    const float gam = a.F.gamma_f64 ? (float)a.F.gamma_f64[i]
-                                    : (float)a.gamma;
-    const float f1[3] = {a.F.e1x[i], a.F.e1y[i], a.F.e1z[i]};
-    const float f2[3] = {a.F.e2x[i], a.F.e2y[i], a.F.e2z[i]};
-    const float d1 = dot3a(rh, f1), d2 = dot3a(rh, f2);
-    const float base = k.amp_pref_j * gam * cos_t * spread * att_f;
+    const float d1 = dot3a(rh, f.e1), d2 = dot3a(rh, f.e2);
+    const float base = k.amp_pref_j * f.gam * cos_t * spread * G.att;
     float amp = base * fa * sinc32(k.kj * d1) * sinc32(k.kj * d2);
     if (!PLAIN && a.taper) {
+      // tan^2 from sin^2 = |rh x n|^2: the narrow taper multiplies a
+      // relative error of 1 - cos^2 by hundreds
       const float ct = fminf(fmaxf(cos_t, (float)kCMin), 1.0f);
-      const float ct2 = ct * ct;
-      amp *= __expf(-__fdividef(1.0f - ct2, ct2) * k.taper_inv);
+      const float sx = __fmaf_rn(rh[1], f.n[2], -rh[2] * f.n[1]);
+      const float sy = __fmaf_rn(rh[2], f.n[0], -rh[0] * f.n[2]);
+      const float sz = __fmaf_rn(rh[0], f.n[1], -rh[1] * f.n[0]);
+      const float s2 = __fmaf_rn(sz, sz, __fmaf_rn(sy, sy, sx * sx));
+      amp *= __expf(-__fdividef(s2, ct * ct) * k.taper_inv);
     }
     float cr = amp, ci = 0.0f;
     float dcr = 0.0f, dci = 0.0f;  // d (cr, ci) / d sigma (GRAD)
     if (ROUGH != SS_ROUGH_NONE) {
-      const float sg = a.F.sigma ? a.F.sigma[i] : k.sigma;
-      const float lc = a.F.corr ? a.F.corr[i] : k.corr;
-      const float l1 = sqrtf(dot3a(f1, f1)), l2 = sqrtf(dot3a(f2, f2));
+      const float sg = f.sg, lc = f.lc, l1 = f.l1, l2 = f.l2;
       const float kk = 2.0f * k.kj * cos_t;
       float dpdx = 0.0f;
       const float dp =
@@ -999,13 +1021,13 @@ __device__ __forceinline__ bool pair_eval(
       if (fa > 0.0f) {
         const float sq = sqrtf(dp);
         const float ai = base * sq;
-        cr += ai * a.F.phasor[2 * i];
-        ci += ai * a.F.phasor[2 * i + 1];
+        cr += ai * f.phr;
+        ci += ai * f.phi;
         if (GRAD && sq > 0.0f) {
           // d sqrt(D) / d sigma = D'(x) 2 sigma K^2 / (2 sqrt(D))
           const float dai = base * dpdx * sg * kk * kk / sq;
-          dcr += dai * a.F.phasor[2 * i];
-          dci = dai * a.F.phasor[2 * i + 1];
+          dcr += dai * f.phr;
+          dci = dai * f.phi;
         }
       }
     }
@@ -1016,14 +1038,14 @@ __device__ __forceinline__ bool pair_eval(
                        (float)a.F.diffuse_amp[i] * ct *
                        (ct > 0.0f ? __powf(ct, 0.5f * k.n_exp)
                                   : (k.n_exp == 0.0f ? 1.0f : 0.0f)) *
-                       spread * att_f;
+                       spread * G.att;
       cr += ad * a.F.diffuse_phasor[2 * i];
       ci += ad * a.F.diffuse_phasor[2 * i + 1];
     }
     // carrier phase 2 k0 opl mod 2 pi (double-float, Cody-Waite)
     float ph, pe;
-    two_prod(k.K2h, opl.hi, ph, pe);
-    const float pl = pe + __fmaf_rn(k.K2h, opl.lo, k.K2l * opl.hi);
+    two_prod(k.K2h, G.opl.hi, ph, pe);
+    const float pl = pe + __fmaf_rn(k.K2h, G.opl.lo, k.K2l * G.opl.hi);
     const float n2 = rintf(ph * 0.159154943091895336f);
     float red = __fmaf_rn(-n2, 6.28318548202514648f, ph);  // exact
     red = __fmaf_rn(-n2, -1.74845553146951e-07f, red) + pl;
@@ -1037,45 +1059,131 @@ __device__ __forceinline__ bool pair_eval(
       pg->gim = gcr * cs + gci * sn;
       pg->sre = dcr * sn - dci * cs;
       pg->sim = dcr * cs + dci * sn;
-      pg->dloss = P.dloss + s_j * (k.att_mask[nj] * 1e-3f);
+      pg->dloss = G.dloss;
     }
   } else {
     const float aa = fa * cos_t * spread;
-    re = aa * aa * att_f * att_f;
+    re = aa * aa * G.att * G.att;
     im = 0.0f;
     pwr = re;
   }
   // fast-time bin u = opl A - B (double-float), float64 path near edges
+  const float nsf = (float)a.n_samples;
   float up, ue, us, ue2;
-  two_prod(opl.hi, k.Ah, up, ue);
+  two_prod(G.opl.hi, k.Ah, up, ue);
   two_sum(up, -k.Bh, us, ue2);
-  const float ul = (ue2 + ue) + __fmaf_rn(opl.hi, k.Al, opl.lo * k.Ah) - k.Bl;
+  const float ul =
+      (ue2 + ue) + __fmaf_rn(G.opl.hi, k.Al, G.opl.lo * k.Ah) - k.Bl;
   float fb = floorf(us);
   float frac = (us - fb) + ul;
   if (frac < 0.0f) { fb -= 1.0f; frac += 1.0f; }
   else if (frac >= 1.0f) { fb += 1.0f; frac -= 1.0f; }
   if ((frac < k.bin_guard || frac > 1.0f - k.bin_guard) && us > -4.0f &&
       us < nsf + 4.0f) {
-    if (!EXACT) return false;
-    bool v64;
-    const double q64[3] = {q[0], q[1], q[2]};
-    const double o64 = full_opl64<NI>(a, p64, q64, v64);
-    const double twtt = __ddiv_rn(__dmul_rn(2.0, o64), a.c);
-    fb = (float)floor(__ddiv_rn(__dsub_rn(twtt, a.t0), a.dt));
+    if (!exact_bin(fb)) return false;
   }
   o.re = re;
   o.im = im;
   o.pwr = pwr;
   o.bin = -1;
-  if (P.valid && fb >= 0.0f && fb < nsf) {
+  if (G.valid && fb >= 0.0f && fb < nsf) {
     int b = (int)fb;
-    if (!PLAIN && a.split) {
-      const float v[3] = {q[0] - T.ph[0], q[1] - T.ph[1], q[2] - T.ph[2]};
-      if (dot3a(v, u) > 0.0f) b += a.n_samples;
-    }
+    if (!PLAIN && a.split && dot3a(v, u) > 0.0f) b += a.n_samples;
     o.bin = b;
   }
   return true;
+}
+
+// Geometry of a solved multi-leg path: final leg, spreading, attenuation.
+__device__ __forceinline__ void path_geo(const RefArgs &a,
+                                         const RefSplitConsts &k,
+                                         const PathS &P, bool grad,
+                                         PairGeo &G) {
+  const int nj = a.leg_last;
+  const float n0 = k.n_leg[0], njn = k.n_leg[nj];
+  G.opl = df_add(P.opl, df_mul(P.s_last, df_make(k.n_leg[nj],
+                                                 k.n_leg_lo[nj])));
+  const float s_j = P.s_last.hi;
+  const float loss = P.loss_db + s_j * (k.att_leg[nj] * 1e-3f);
+  const float sperp = P.sum_perp + s_j / njn;
+  const float spar = P.sum_par + s_j / (njn * P.c_last * P.c_last);
+  const float l_perp = n0 * sperp;
+  const float l_par = n0 * P.c0 * P.c0 * spar;
+  const float flux = (n0 * P.c0) / (njn * P.c_last);
+  G.att = exp2f(-loss * 0.33219280949f);  // 10^(-loss/10)
+  G.spread = P.tau2 * flux / (l_par * l_perp);
+  for (int j = 0; j < 3; ++j) {
+    G.rh[j] = P.rh[j];
+    G.d0[j] = P.d0[j];
+  }
+  G.dloss = grad ? P.dloss + s_j * (k.att_mask[nj] * 1e-3f) : 0.0f;
+  G.valid = P.valid;
+}
+
+template <int NI, int ROUGH, bool EXACT, bool GRAD = false,
+          bool PLAIN = false>
+__device__ __forceinline__ bool pair_eval(
+    const RefArgs &a, const RefSplitConsts &k, const TraceS &T,
+    const double *p64, const float *u, const float *pv, const float *pat,
+    int pa_len, const float *lg, const float *fad, int i, const float *q,
+    PairOut &o, PairGrad *pg = nullptr) {
+  PathS P;
+  if (NI <= 0)
+    path_sequential_split<EXACT, GRAD>(a, k, T, p64, q, P);
+  else
+    path_joint_split<NI <= 0 ? 1 : NI, EXACT, GRAD>(a, k, T, p64, q, P);
+  if (!EXACT && P.defer) return false;
+  PairGeo G;
+  path_geo(a, k, P, GRAD, G);
+  FacetS f;
+  load_facet<ROUGH>(a, k, i, f);
+  const float v[3] = {q[0] - T.ph[0], q[1] - T.ph[1], q[2] - T.ph[2]};
+  return pair_finish<ROUGH, GRAD, PLAIN>(
+      a, k, f, G, v, u, pv, pat, pa_len, lg, fad, i, o, pg, [&](float &fb) {
+        if (!EXACT) return false;
+        bool v64;
+        const double q64[3] = {q[0], q[1], q[2]};
+        const double o64 = full_opl64<NI <= 0 ? 0 : NI>(a, p64, q64, v64);
+        const double twtt = __ddiv_rn(__dmul_rn(2.0, o64), a.c);
+        fb = (float)floor(__ddiv_rn(__dsub_rn(twtt, a.t0), a.dt));
+        return true;
+      });
+}
+
+// The single-crossing pair (kOneNI) of a facet whose record and mean-plane
+// constants the caller holds, against the trace staged at `tr` (position hi
+// and lo); false when it needs a float64 decision.
+template <int ROUGH, bool GRAD, bool PLAIN>
+__device__ __forceinline__ bool pair_one(
+    const RefArgs &a, const RefSplitConsts &k, const float4 *tr,
+    const float *u, const float *pv, const float *pat, int pa_len,
+    const float *lg, const float *fad, int i, const FacetS &f,
+    const OneFacet &m, PairOut &o, PairGrad *pg = nullptr) {
+  float Ph[3], Pl[3];
+  const float4 A = tr[0];
+  one_offset(A, make_float2(tr[1].x, tr[1].y), f.q, Ph, Pl);
+  int cell;
+  if (!one_cell(k.one, m, Ph, a.ifc[0].ny, a.ifc[0].nx, kLookupGuard, cell))
+    return false;
+  PairGeo G;
+  one_path<GRAD>(k.one, k.legs, a.ifc[0].table, cell, f.q, Ph, Pl, kTol32,
+                 G);
+  if (a.rough_cross) {
+    // c0 and c_last of the crossing again (a rarely used option)
+    const float is2 = rsqrtf(fmaxf(dot3a(G.d0, G.d0), 1e-30f));
+    const float *t = a.ifc[0].table + (size_t)cell * 6 + 3;
+    const float in = rsqrtf(dot3a(t, t));
+    const float c1 = fabsf(dot3a(G.d0, t)) * in * is2;
+    const float c2 = fabsf(dot3a(G.rh, t)) * in;
+    const float kt = k.k0 * (k.legs.n1 * fmaxf(c1, (float)kCMin) -
+                             k.legs.n2 * c2);
+    const float sk = k.sig_c[0] * kt;
+    G.spread *= __expf(-2.0f * sk * sk);
+  }
+  const float v[3] = {-Ph[0], -Ph[1], -Ph[2]};
+  return pair_finish<ROUGH, GRAD, PLAIN>(a, k, f, G, v, u, pv, pat, pa_len,
+                                         lg, fad, i, o, pg,
+                                         [](float &) { return false; });
 }
 
 // One CTA's work item of the fast kernel: facet chunk `chunk` of trace
@@ -1092,6 +1200,7 @@ __device__ __forceinline__ void refracted_split_cta(const RefArgs &a,
   float *lg = reinterpret_cast<float *>(hist + (size_t)a.tb * a.n_seg);
   __shared__ double s_p64[SS_MAX_TB][3];
   __shared__ TraceS s_tr[SS_MAX_TB];
+  __shared__ float4 s_t4[SS_MAX_TB][2];  // position hi, lo (kOneNI)
   __shared__ float s_u[SS_MAX_TB][3], s_pv[SS_MAX_TB][6];
   __shared__ int s_lo[SS_MAX_TB], s_hi[SS_MAX_TB];
   __shared__ float s_drop[SS_MAX_TB];
@@ -1107,6 +1216,7 @@ __device__ __forceinline__ void refracted_split_cta(const RefArgs &a,
   if (tid < nt) {
     const int t = t_base + tid;
     load_trace(a, t, s_tr[tid], s_p64[tid], s_u[tid], s_pv[tid]);
+    if (NI == kOneNI) stage_trace4(s_tr[tid], s_t4[tid]);
     long lo = (long)a.off[t] * a.bs;
     long hi = min((long)(a.off[t] + a.n_win) * a.bs, (long)a.N);
     s_lo[tid] = (int)min(lo, (long)a.N);
@@ -1147,13 +1257,26 @@ __device__ __forceinline__ void refracted_split_cta(const RefArgs &a,
     if (base >= i_end) break;
     const int i = base + lane;
     if (i >= i_end) continue;
-    const float q[3] = {a.F.cx[i], a.F.cy[i], a.F.cz[i]};
+    FacetS f;
+    OneFacet m;
+    f.q[0] = a.F.cx[i]; f.q[1] = a.F.cy[i]; f.q[2] = a.F.cz[i];
+    if (NI == kOneNI) {
+      load_facet<ROUGH>(a, k, i, f);
+      one_facet(k.one, f.q, m);
+    }
     for (int tt = 0; tt < nt; ++tt) {
       if (i < s_lo[tt] || i >= s_hi[tt]) continue;
       PairOut o;
-      if (!pair_eval<NI, ROUGH, false, false, PLAIN>(
-              a, k, s_tr[tt], s_p64[tt], s_u[tt], s_pv[tt], s_pat, pa_len,
-              lg, s_fad, i, q, o)) {
+      bool ok;
+      if (NI == kOneNI)
+        ok = pair_one<ROUGH, false, PLAIN>(a, k, s_t4[tt], s_u[tt], s_pv[tt],
+                                           s_pat, pa_len, lg, s_fad, i, f, m,
+                                           o);
+      else
+        ok = pair_eval<NI, ROUGH, false, false, PLAIN>(
+            a, k, s_tr[tt], s_p64[tt], s_u[tt], s_pv[tt], s_pat, pa_len, lg,
+            s_fad, i, f.q, o);
+      if (!ok) {
         const unsigned long long bit =
             (unsigned long long)(t_base + tt) * a.defer_w + (i - s_lo[tt]);
         atomicOr(&a.defer_mask[bit >> 5], 1u << (bit & 31));
@@ -1473,6 +1596,7 @@ refracted_batch_fixup(const RefBatchJob *jobs, int n_jobs,
   int refracted_batch_occupancy_ni##N(int rough_kind, bool plain,          \
                                       size_t smem);
 SS_REF_BATCH_DECL(0)
+SS_REF_BATCH_DECL(one)
 SS_REF_BATCH_DECL(1)
 SS_REF_BATCH_DECL(2)
 SS_REF_BATCH_DECL(3)
@@ -1558,8 +1682,17 @@ RefSplitConsts split_consts(const RefArgs &a);
 // Dynamic shared memory of the fast kernel for a trace block of tb.
 size_t split_smem_bytes(const RefArgs &a, int tb);
 
+// Whether the call takes the single-crossing path (kOneNI): one crossed
+// interface solved sequentially, the final leg directly below it, and
+// refractive indices that are the roots of the permittivities (the path
+// takes the Fresnel factor from Snell's cosines).
+bool one_crossing(const RefArgs &a);
+
 // Fast + fix-up launches of one crossed-interface count (NI = 0: the
-// sequential path), each instantiated in its own translation unit.
+// sequential path; one: a single crossing), each instantiated in its own
+// translation unit.
+int split_launch_one(RefArgs &a, const RefSplitConsts &k, const Plan &p,
+                     size_t smem, cudaStream_t st);
 int split_launch_ni0(RefArgs &a, const RefSplitConsts &k, const Plan &p,
                      size_t smem, cudaStream_t st);
 int split_launch_ni1(RefArgs &a, const RefSplitConsts &k, const Plan &p,
