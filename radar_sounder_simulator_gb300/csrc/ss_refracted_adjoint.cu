@@ -31,8 +31,6 @@ int refracted_adjoint_launch(RefArgs &a, const AdjArgs &j,
   RefSplitConsts k = split_consts(a);
   for (int m = 0; m <= a.leg_last; ++m)
     k.att_mask[m] = alpha_mask ? (float)alpha_mask[m] : 0.0f;
-  k.legs.m1 = k.att_mask[0] * 1e-3f;
-  k.legs.m2 = k.att_mask[1] * 1e-3f;
   const size_t smem =
       a.rough_kind ? (size_t)(a.n_terms + 1) * sizeof(float) : 0;
   cudaError_t e = cudaMemsetAsync(
@@ -41,8 +39,7 @@ int refracted_adjoint_launch(RefArgs &a, const AdjArgs &j,
   if (a.joint)
     return a.ni <= 2 ? adjoint_launch_joint12(a, k, j, smem, st)
                      : adjoint_launch_joint34(a, k, j, smem, st);
-  return one_crossing(a) ? adjoint_launch_one(a, k, j, smem, st)
-                         : adjoint_launch_ni<0>(a, k, j, smem, st);
+  return adjoint_launch_ni<0>(a, k, j, smem, st);
 }
 
 }  // namespace ss

@@ -29,22 +29,6 @@ constexpr double kLn10 = 2.302585092994045684;
 
 int refracted_adjoint_blocks(int N);
 
-// A pair's terms weighted by the trace's upstream gradient and the forward
-// field of its bin, when that lies in the power window.
-__device__ __forceinline__ void adjoint_add(const RefArgs &a,
-                                            const AdjArgs &j,
-                                            const PairOut &o,
-                                            const PairGrad &pg, int t,
-                                            double g, double &gR, double &gS,
-                                            double &gA) {
-  if (o.bin < j.bin_lo || o.bin >= j.bin_hi) return;
-  const double2 f =
-      reinterpret_cast<const double2 *>(j.field)[(size_t)t * a.n_seg + o.bin];
-  gR += g * (f.x * pg.gre + f.y * pg.gim);
-  gS += g * (f.x * pg.sre + f.y * pg.sim);
-  gA += g * (f.x * o.re + f.y * o.im) * (double)pg.dloss;
-}
-
 // One pair's terms of the three gradients (before the ln10 factors).
 template <int NI, int ROUGH, bool EXACT>
 __device__ __forceinline__ bool adjoint_pair(
@@ -57,7 +41,12 @@ __device__ __forceinline__ bool adjoint_pair(
   if (!pair_eval<NI, ROUGH, EXACT, true>(a, k, T, p64, u, pv, pat, pa_len, lg,
                                         fad, i, q, o, &pg))
     return false;
-  adjoint_add(a, j, o, pg, t, g, gR, gS, gA);
+  if (o.bin < j.bin_lo || o.bin >= j.bin_hi) return true;
+  const double2 f =
+      reinterpret_cast<const double2 *>(j.field)[(size_t)t * a.n_seg + o.bin];
+  gR += g * (f.x * pg.gre + f.y * pg.gim);
+  gS += g * (f.x * pg.sre + f.y * pg.sim);
+  gA += g * (f.x * o.re + f.y * o.im) * (double)pg.dloss;
   return true;
 }
 
@@ -87,13 +76,12 @@ __device__ __forceinline__ void adjoint_stage_tables(const RefArgs &a,
 // several (chosen so the grid fills whole waves) each part adds them to
 // outputs the launch has zeroed.
 template <int NI, int ROUGH>
-__global__ void __launch_bounds__(kAdjThreads, NI <= 0 ? 6 : 1)
+__global__ void __launch_bounds__(kAdjThreads, NI == 0 ? 6 : 1)
 refracted_adjoint_kernel(RefArgs a, RefSplitConsts k, AdjArgs j) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float *lg = reinterpret_cast<float *>(smem_raw);
   __shared__ double s_p64[kAdjTB][3];
   __shared__ TraceS s_tr[kAdjTB];
-  __shared__ float4 s_t4[kAdjTB][2];
   __shared__ float s_u[kAdjTB][3], s_pv[kAdjTB][6];
   __shared__ int s_lo[kAdjTB], s_hi[kAdjTB];
   __shared__ double s_g[kAdjTB];
@@ -106,17 +94,11 @@ refracted_adjoint_kernel(RefArgs a, RefSplitConsts k, AdjArgs j) {
   const int i_last = min(i_first + kAdjThreads, a.N) - 1;
   int pa_len;
   adjoint_stage_tables<ROUGH>(a, s_pat, s_fad, lg, pa_len);
-  FacetS f;
-  OneFacet m;
-  f.q[0] = f.q[1] = f.q[2] = 0.0f;
+  float q[3] = {0.0f, 0.0f, 0.0f};
   if (i < a.N) {
-    f.q[0] = a.F.cx[i];
-    f.q[1] = a.F.cy[i];
-    f.q[2] = a.F.cz[i];
-    if (NI == kOneNI) {
-      load_facet<ROUGH>(a, k, i, f);
-      one_facet(k.one, f.q, m);
-    }
+    q[0] = a.F.cx[i];
+    q[1] = a.F.cy[i];
+    q[2] = a.F.cz[i];
   }
   const int parts = gridDim.y;
   const int t_begin = (int)((long)a.T * blockIdx.y / parts);
@@ -128,7 +110,6 @@ refracted_adjoint_kernel(RefArgs a, RefSplitConsts k, AdjArgs j) {
     if (tid < nt) {
       const int t = t0 + tid;
       load_trace(a, t, s_tr[tid], s_p64[tid], s_u[tid], s_pv[tid]);
-      if (NI == kOneNI) stage_trace4(s_tr[tid], s_t4[tid]);
       const long lo = (long)a.off[t] * a.bs;
       const long hi = min((long)(a.off[t] + a.n_win) * a.bs, (long)a.N);
       s_lo[tid] = (int)min(lo, (long)a.N);
@@ -141,20 +122,9 @@ refracted_adjoint_kernel(RefArgs a, RefSplitConsts k, AdjArgs j) {
       if (s_hi[tt] <= i_first || s_lo[tt] > i_last || s_g[tt] == 0.0)
         continue;
       if (i >= a.N || i < s_lo[tt] || i >= s_hi[tt]) continue;
-      bool ok;
-      if (NI == kOneNI) {
-        PairOut o;
-        PairGrad pg;
-        ok = pair_one<ROUGH, true, false>(a, k, s_t4[tt], s_u[tt], s_pv[tt],
-                                          s_pat, pa_len, lg, s_fad, i, f, m,
-                                          o, &pg);
-        if (ok) adjoint_add(a, j, o, pg, t0 + tt, s_g[tt], gR, gS, gA);
-      } else {
-        ok = adjoint_pair<NI, ROUGH, false>(
-            a, k, j, s_tr[tt], s_p64[tt], s_u[tt], s_pv[tt], s_pat, pa_len,
-            lg, s_fad, t0 + tt, i, f.q, s_g[tt], gR, gS, gA);
-      }
-      if (!ok) {
+      if (!adjoint_pair<NI, ROUGH, false>(a, k, j, s_tr[tt], s_p64[tt], s_u[tt],
+                                      s_pv[tt], s_pat, pa_len, lg, s_fad,
+                                      t0 + tt, i, q, s_g[tt], gR, gS, gA)) {
         const unsigned long long bit =
             (unsigned long long)(t0 + tt) * a.N + i;
         atomicOr(&j.defer_mask[bit >> 5], 1u << (bit & 31));
@@ -319,10 +289,6 @@ inline int adjoint_launch_ni(RefArgs &a, const RefSplitConsts &k,
       return adjoint_launch_r<NI, SS_ROUGH_EXP_AREA>(a, k, j, smem, st);
   }
 }
-
-// Single-crossing adjoint launches (ss_refracted_adjoint_one.cu).
-int adjoint_launch_one(RefArgs &a, const RefSplitConsts &k, const AdjArgs &j,
-                       size_t smem, cudaStream_t st);
 
 // Joint-path adjoint launches through 1-2 and 3-4 interfaces
 // (ss_refracted_adjoint_joint12.cu, ss_refracted_adjoint_joint34.cu).

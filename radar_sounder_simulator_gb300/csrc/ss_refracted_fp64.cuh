@@ -271,9 +271,12 @@ static __device__ __noinline__ void joint64(
     const double (&Nn)[NI][3], const double *nm, int n_newton,
     int n_backtrack, double (&X)[NI][3], double (&cinc)[NI],
     double (&cout_)[NI], double (&S)[NI + 1], bool &valid, int ni = NI) {
-  double pq[3] = {p[0] - q[0], p[1] - q[1], p[2] - q[2]};
-  const double scale = fmax(sqrt(dot3v(pq, pq)), kTiny);
-  const double inv = 1.0 / scale;
+  // the path scale as a power of two: scaling rounds nothing
+  const float pq[3] = {(float)(p[0] - q[0]), (float)(p[1] - q[1]),
+                       (float)(p[2] - q[2])};
+  const int ex = ilogbf(fmaxf(
+      sqrtf(pq[0] * pq[0] + pq[1] * pq[1] + pq[2] * pq[2]), 1e-30f));
+  const double scale = ldexp(1.0, ex), inv = ldexp(1.0, -ex);
   // in-plane bases (refraction_joint.py:196-204), segment bases and the
   // offsets of the chain of two-point solves (refraction.py) that starts
   // the joint solve

@@ -59,7 +59,10 @@ RefSplitConsts split_consts(const RefArgs &a) {
     }
     const double n1 = a.n_leg[0], n2 = a.n_leg[1];
     O.up = n1 <= n2;
-    O.r = (float)(std::min(n1, n2) / std::max(n1, n2));
+    const double r = std::min(n1, n2) / std::max(n1, n2);
+    O.r = (float)r;
+    O.k2 = (float)(-0.5 * (1.0 - r * r));
+    O.k4 = (float)(-0.125 * (1.0 - r * r) * (1.0 + 3.0 * r * r));
     O.vec = (reinterpret_cast<uintptr_t>(I.table) & 7) == 0;
     OneLegs &l = k.legs;
     const df d1 = df_from_double(n1), d2 = df_from_double(n2);
@@ -109,6 +112,7 @@ RefSplitConsts split_consts(const RefArgs &a) {
 
 bool one_crossing(const RefArgs &a) {
   if (a.joint || a.ni != 1 || a.leg_last != 1) return false;
+  if (a.F.gamma_f64 && a.F.sigma) return false;
   for (int i = 0; i < 2; ++i)
     if (!(std::fabs(a.n_leg[i] * a.n_leg[i] - a.eps_leg[i]) <=
           1e-9 * a.eps_leg[i]))
