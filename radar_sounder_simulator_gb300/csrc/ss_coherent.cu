@@ -74,7 +74,11 @@ __device__ __forceinline__ void coherent_fp64_cta(const CoArgs &a, int chunk,
   __syncthreads();
 
   const double k = a.k;
-  const double amp_pref = k / kTwoPi;
+  const double amp_pref = k / kTwoPi, k_pi = k / kPi;
+  const double taper_i = a.taper ? -1.0 / (2.0 * a.taper_s * a.taper_s) : 0.0;
+  // fast-time bin u = r bA - bB; the reference's own chain decides a pair
+  // within 1e-8 bins of an edge (the two differ by ~1e-11 bins)
+  const double bA = 2.0 / (a.c * a.dt), bB = a.t0 / a.dt;
   // traces rotated across lanes and dropped power kept per thread, as in
   // the split form (ss_coherent_split.cu)
   const int rot = (tid & 31) % max(nt, 1);
@@ -88,28 +92,30 @@ __device__ __forceinline__ void coherent_fp64_cta(const CoArgs &a, int chunk,
     const double e2x = a.F.e2x[i], e2y = a.F.e2y[i], e2z = a.F.e2z[i];
     const double area = a.F.area[i];
     const double gam = a.F.gamma_f32 ? (double)a.F.gamma_f32[i] : a.gamma;
+    const double pref = amp_pref * gam * area;
     for (int st = 0; st < nt; ++st) {
       const int tt = rot + st < nt ? rot + st : rot + st - nt;
       if (i < s_lo[tt] || i >= s_hi[tt]) continue;
-      // range chain in round-to-nearest (bins bit-identical to NumPy)
+      // the squared range in round-to-nearest (the reference's rounding);
+      // one reciprocal root serves the range and every quotient by it
       const double dx = __dsub_rn(s_p[tt][0], cx);
       const double dy = __dsub_rn(s_p[tt][1], cy);
       const double dz = __dsub_rn(s_p[tt][2], cz);
       const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx),
                                             __dmul_rn(dy, dy)),
                                   __dmul_rn(dz, dz));
-      const double r = __dsqrt_rn(r2);
-      const double cosv = dot3(dx, dy, dz, nx, ny, nz) / r;
-      const double rx = dx / r, ry = dy / r, rz = dz / r;
-      const double d1 = dot3(rx, ry, rz, e1x, e1y, e1z);
-      const double d2 = dot3(rx, ry, rz, e2x, e2y, e2z);
-      const double s1 = sinc_np(d1 * (k / kPi));
-      const double s2 = sinc_np(d2 * (k / kPi));
-      double amp = amp_pref * gam * cosv * area * s1 * s2 / (r * r);
+      const double ir = rsqrt(r2);
+      double r = r2 * ir;
+      r = fma(fma(-r, r, r2), 0.5 * ir, r);
+      const double cosv = dot3(dx, dy, dz, nx, ny, nz) * ir;
+      const double d1 = dot3(dx, dy, dz, e1x, e1y, e1z) * ir;
+      const double d2 = dot3(dx, dy, dz, e2x, e2y, e2z) * ir;
+      const double ir2 = ir * ir;
+      double amp = pref * cosv * sinc2_np(d1 * k_pi, d2 * k_pi) * ir2;
       if (a.taper) {
         double cc = fmin(fmax(cosv, 1e-9), 1.0);
         double c2 = cc * cc;
-        amp *= exp(-(1.0 - c2) / (c2 * (2.0 * a.taper_s * a.taper_s)));
+        amp *= exp((1.0 - c2) / c2 * taper_i);
       }
       double cr = amp, ci = 0.0;
       if (a.rough_kind != SS_ROUGH_NONE) {
@@ -122,7 +128,7 @@ __device__ __forceinline__ void coherent_fp64_cta(const CoArgs &a, int chunk,
                                   a.fad.L, sg, lc, kk, 2.0 * k * d1 / l1,
                                   2.0 * k * d2 / l2, l1, l2);
         const double amp_i =
-            area > 0.0 ? amp_pref * gam * cosv / (r * r) * sqrt(dp) : 0.0;
+            area > 0.0 ? amp_pref * gam * cosv * ir2 * sqrt(dp) : 0.0;
         const double sk = sg * kk;
         const double att = exp(-0.5 * (sk * sk));
         const double phr = a.F.phasor[2 * i], phi = a.F.phasor[2 * i + 1];
@@ -136,13 +142,19 @@ __device__ __forceinline__ void coherent_fp64_cta(const CoArgs &a, int chunk,
       double im = cr * cs + ci * sn;
       if (a.pat_kind != SS_PAT_ISOTROPIC) {
         const double g = gain64(a.pat_kind, a.pat_n, a.pa, a.pb, s_pv[tt],
-                                -rx, -ry, -rz);
+                                -dx * ir, -dy * ir, -dz * ir);
         re *= g * g;
         im *= g * g;
       }
-      // fast-time bin (geometry.py:18-24), round-to-nearest like NumPy
-      const double twtt = __ddiv_rn(__dmul_rn(2.0, r), a.c);
-      const double u = __ddiv_rn(__dsub_rn(twtt, a.t0), a.dt);
+      // fast-time bin (geometry.py:18-24)
+      double u = fma(r, bA, -bB);
+      double fb = floor(u);
+      if (fabs(u - rint(u)) < 1e-8) {
+        const double rd = __dsqrt_rn(r2);
+        const double twtt = __ddiv_rn(__dmul_rn(2.0, rd), a.c);
+        u = __ddiv_rn(__dsub_rn(twtt, a.t0), a.dt);
+        fb = floor(u);
+      }
       int side_off = 0;
       if (a.split) {
         const double ax = -dx, ay = -dy, az = -dz;  // c - p
@@ -150,7 +162,6 @@ __device__ __forceinline__ void coherent_fp64_cta(const CoArgs &a, int chunk,
           side_off = a.n_samples;
       }
       double2 *h = hist + (size_t)tt * a.n_seg + side_off;
-      const double fb = floor(u);
       if (a.interp) {
         const double w = __dsub_rn(u, fb);
         const double parts[2] = {1.0 - w, w};
@@ -259,11 +270,18 @@ int coherent_plan(const ss_coherent_opts *o, int T, int N, Plan *p,
   int tb = (int)std::max<size_t>(1, std::min<size_t>(budget / per_trace,
                                                      SS_MAX_TB));
   tb = std::min(tb, T);
-  p->tb = tb;
-  p->n_groups = (T + tb - 1) / tb;
   p->threads = fp64 || rough ? 256 : 512;
   const long window = std::min<long>((long)o->n_win * o->block_size, N);
-  const int max_chunks = (int)std::max<long>(1, window / 512);
+  // a chunk gives every thread of its CTA a facet (256-thread CTAs at least
+  // one, 512-thread ones half of them); a call too small to cover the SMs
+  // takes smaller trace blocks until it does (64^2 facets x 32 traces of
+  // 512 bins ran on 32 of 152 SMs)
+  const int max_chunks = (int)std::max<long>(1, window / 256);
+  while (tb > (fp64 ? 1 : 2) &&
+         (long)((T + tb - 1) / tb) * max_chunks < 2L * sm_count())
+    tb = (tb + 1) / 2;
+  p->tb = tb;
+  p->n_groups = (T + tb - 1) / tb;
   // resident CTAs per SM: 2 (512-thread smooth split, 96 KB FP64), 3
   // (rough split at 80 registers); the chunk count whose item total fills
   // 1-4 whole waves best (a last wave a tenth full costs a full wave); on

@@ -90,8 +90,7 @@ __device__ __forceinline__ double gain64(int kind, int n, const double *pa, cons
   switch (kind) {
     case SS_PAT_DIPOLE: {
       double ca = dot3(dx, dy, dz, pv[0], pv[1], pv[2]);
-      double s = sqrt(fmax(1.0 - ca * ca, 1e-12));
-      return cos((kPi / 2.0) * ca) / s;
+      return cospi(0.5 * ca) * rsqrt(fmax(1.0 - ca * ca, 1e-12));
     }
     case SS_PAT_ARRAY: {
       double ne = pa[0];
