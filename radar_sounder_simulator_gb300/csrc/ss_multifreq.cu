@@ -29,6 +29,7 @@
 
 #include "ss_df.cuh"
 #include "ss_f32.cuh"
+#include "ss_f32x2.cuh"
 
 namespace ss {
 
@@ -47,10 +48,17 @@ struct MfArgs {
   void *part;
 };
 
-// split form: 128 threads x 8 frequencies = 1024 frequencies per CTA,
-// 4 traces per CTA, tiles of 32 facets (4 x 32 = one pair per thread)
-constexpr int kMfThreads = 128, kMfF = 8, kMfTB = 4, kMfP = 32;
-constexpr int kMfFBlock = kMfThreads * kMfF;
+// split form: 1024 frequencies and 4 traces per CTA, tiles of 32 facets (4 x
+// 32 = one pair per thread). Half of the CTA's threads take two of the
+// traces, each thread 16 frequencies as two interleaved chains of 8 -- one
+// packed instruction advances both -- so the carrier phase's head (product,
+// reduction, sine and cosine) is paid once per 16 and a chain is as long as
+// the 8 frequencies a float32 step may drift over.
+constexpr int kMfThreads = 128, kMfF = 16, kMfTB = 4, kMfP = 32;
+constexpr int kMfHalf = kMfThreads / 2, kMfTB2 = kMfTB / 2;
+constexpr int kMfFBlock = kMfHalf * kMfF;
+// FP64 form: 128 threads x 8 frequencies
+constexpr int kMf64F = 8;
 // FP64 form: 2 traces per CTA, tiles of 64 facets
 constexpr int kMf64TB = 2, kMf64P = 64;
 
@@ -62,18 +70,6 @@ struct MfSplitConsts {
   float kf1, dk;    // wavenumber of the first frequency and the step
   float gamma, taper_inv, fadL, sigma, corr;
 };
-
-// Compensated float sum: value = s + c (two-sum error terms gathered in c).
-struct Acc2 {
-  float s, c;
-};
-
-__device__ __forceinline__ void acc2_add(Acc2 &a, float x) {
-  float s, e;
-  two_sum(a.s, x, s, e);
-  a.s = s;
-  a.c += e;
-}
 
 // x * y of a double-float and a double-float, rounded to a double-float.
 __device__ __forceinline__ void df_prod(float xh, float xl, float yh, float yl,
@@ -89,6 +85,37 @@ __device__ __forceinline__ float reduce_df_2pi(float hi, float lo) {
   const float n = rintf(hi * 0.159154943091895336f);
   float r = __fmaf_rn(-n, 6.28318548202514648f, hi);  // exact
   return __fmaf_rn(-n, -1.74845553146951e-07f, r) + lo;
+}
+
+// Sine and cosine of hi + lo (|hi| up to ~1e5) to a float32 ulp or so: the
+// argument is reduced to [-pi/4, pi/4] by quarter turns (the first product
+// exact: hi and n c share their leading bits), then the minimax polynomials
+// of Moshier's Cephes library (sinf.c) run on it, without the library
+// call's large-argument branch.
+__device__ __forceinline__ void sincos_df(float hi, float lo, float &sn,
+                                          float &cs) {
+  if (fabsf(hi) > 6e6f) {  // quarter turns beyond the integer trick: whole
+    const float m = rintf(hi * 0.159154943091895336f);  // turns first
+    hi = __fmaf_rn(-m, 6.28318548202514648f, hi);
+    lo = __fmaf_rn(m, 1.74845553146951e-07f, lo);
+  }
+  const float t = __fmaf_rn(hi, 0.636619772367581343f, 12582912.0f);
+  const int q = __float_as_int(t);
+  const float n = t - 12582912.0f;
+  float y = __fmaf_rn(-n, 1.57079637050628662f, hi);
+  y = __fmaf_rn(n, 4.37113900018624283e-8f, y) + lo;
+  const float z = y * y;
+  const float s = __fmaf_rn(
+      __fmaf_rn(__fmaf_rn(-1.9515295891e-4f, z, 8.3321608736e-3f), z,
+                -1.6666654611e-1f) * z, y, y);
+  const float c = __fmaf_rn(
+      __fmaf_rn(__fmaf_rn(2.443315711809948e-5f, z, -1.388731625493765e-3f),
+                z, 4.166664568298827e-2f) * z, z, __fmaf_rn(-0.5f, z, 1.0f));
+  const bool odd = q & 1;
+  sn = odd ? c : s;
+  cs = odd ? s : c;
+  sn = __int_as_float(__float_as_int(sn) ^ ((q & 2) << 30));
+  cs = __int_as_float(__float_as_int(cs) ^ (((q + 1) & 2) << 30));
 }
 
 // sin(x)/x to float32 accuracy for any x: the full-amplitude form evaluates
@@ -122,9 +149,11 @@ multifreq_split_kernel(MfArgs a, MfSplitConsts k) {
   __shared__ int s_lo[kMfTB], s_hi[kMfTB];
   __shared__ int s_rng[2];
   __shared__ float s_fad[SS_FAD_N];
-  // pair data: R (hi, lo), amplitude (re, im) or (g, -), d1, d2, step (re, im)
+  // pair data: R (hi, lo), amplitude (re, im) or (g, -); step (re, im) of
+  // one and of two frequencies; d1, d2 (full amplitudes)
   __shared__ float4 s_pa[kMfTB * kMfP];
   __shared__ float4 s_pb[kMfTB * kMfP];
+  __shared__ float2 s_pd[FULL ? kMfTB * kMfP : 1];
   const int chunk = blockIdx.x;
   const int t_base = blockIdx.y * kMfTB;
   const int nt = min(kMfTB, a.T - t_base);
@@ -158,7 +187,8 @@ multifreq_split_kernel(MfArgs a, MfSplitConsts k) {
   __syncthreads();
 
   // this thread's first frequency index and its frequency / wavenumber
-  const int kn = blockIdx.z * kMfFBlock + tid * kMfF;
+  const int half = tid / kMfHalf;
+  const int kn = blockIdx.z * kMfFBlock + (tid % kMfHalf) * kMfF;
   float fsh, fsl;
   {
     float p, e;
@@ -169,18 +199,21 @@ multifreq_split_kernel(MfArgs a, MfSplitConsts k) {
     fast_two_sum(s, e2 + e + k.f1l, fsh, fsl);
   }
   const float ks = __fmaf_rn((float)kn, k.dk, k.kf1);
-  float2 acc[kMfTB][kMfF];
+  // re and im sums of this half's traces, frequencies (2q, 2q + 1) packed
+  float2 accr[kMfTB2][kMfF / 2], acci[kMfTB2][kMfF / 2];
 #pragma unroll
-  for (int tt = 0; tt < kMfTB; ++tt)
+  for (int tt = 0; tt < kMfTB2; ++tt)
 #pragma unroll
-    for (int q = 0; q < kMfF; ++q) acc[tt][q] = make_float2(0.0f, 0.0f);
+    for (int q = 0; q < kMfF / 2; ++q)
+      accr[tt][q] = acci[tt][q] = make_float2(0.0f, 0.0f);
 
   for (int base = s_rng[0]; base < s_rng[1]; base += kMfP) {
     // --- phase A: one (trace, facet) pair per thread ---
     {
       const int tt = tid / kMfP, i = base + tid % kMfP;
       float4 pa = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      float4 pb = make_float4(1.0f, 0.0f, 0.0f, 0.0f);
+      float4 pb = make_float4(1.0f, 0.0f, 1.0f, 0.0f);
+      float2 pd = make_float2(0.0f, 0.0f);
       if (i < s_rng[1] && i >= s_lo[tt] && i < s_hi[tt]) {
         const float cx = a.F.cx[i], cy = a.F.cy[i], cz = a.F.cz[i];
         float dxh, dxl, dyh, dyl, dzh, dzl, e;
@@ -228,12 +261,14 @@ multifreq_split_kernel(MfArgs a, MfSplitConsts k) {
         // R = 4 pi r / c; phase of frequency f is R f
         float Rh, Rl;
         df_prod(k.Rch, k.Rcl, r.hi, r.lo, Rh, Rl);
-        // step between neighbouring frequencies: exp(-j R df)
+        // steps over one and two frequencies: exp(-j R df), exp(-2j R df)
         float dh, dl;
         df_prod(Rh, Rl, k.dfh, k.dfl, dh, dl);
-        float sn, cs;
+        float sn, cs, sn2, cs2;
         sincosf(reduce_df_2pi(dh, dl), &sn, &cs);
-        pb = make_float4(cs, -sn, d1, d2);
+        sincosf(reduce_df_2pi(2.0f * dh, 2.0f * dl), &sn2, &cs2);
+        pb = make_float4(cs, -sn, cs2, -sn2);
+        pd = make_float2(d1, d2);
         if (FULL) {
           // amplitude (k / 2 pi) g sinc(k d1) sinc(k d2), evaluated per
           // frequency; contribution j amp exp(-j phase)
@@ -266,44 +301,56 @@ multifreq_split_kernel(MfArgs a, MfSplitConsts k) {
       __syncthreads();
       s_pa[tid] = pa;
       s_pb[tid] = pb;
+      if (FULL) s_pd[tid] = pd;
       __syncthreads();
     }
-    // --- phase B: every thread, every pair of the tile, its frequencies ---
+    if (kn >= a.K) continue;  // whole warps past the band's end
+    // --- phase B: every thread, its traces' pairs, its frequencies ---
 #pragma unroll
-    for (int tt = 0; tt < kMfTB; ++tt) {
+    for (int tt = 0; tt < kMfTB2; ++tt) {
       for (int f = 0; f < kMfP; ++f) {
-        const float4 pa = s_pa[tt * kMfP + f];
-        const float4 pb = s_pb[tt * kMfP + f];
+        const int e = (half * kMfTB2 + tt) * kMfP + f;
+        const float4 pa = s_pa[e];
+        const float4 pb = s_pb[e];
         if (pa.z == 0.0f && pa.w == 0.0f) continue;  // outside the window
-        float ph, pl;
-        df_prod(pa.x, pa.y, fsh, fsl, ph, pl);
+        float ph, pe;
+        two_prod(pa.x, fsh, ph, pe);
+        pe = __fmaf_rn(pa.x, fsl, __fmaf_rn(pa.y, fsh, pe));
         // ulp-accurate sincos: the band response sums many partly
         // cancelling phasors, and MUFU's ~4e-7 absolute error would show
         // at -60 dB of the synthesised profile
         float sn, cs;
-        sincosf(reduce_df_2pi(ph, pl), &sn, &cs);
-        float er = cs, ei = -sn;  // exp(-j phase)
-        if (FULL) {
+        sincos_df(ph, pe, sn, cs);
+        // z0 = (amplitude) exp(-j phase), z1 = z0 step; both then advance
+        // by two frequencies at a time
+        float z0r = cs, z0i = -sn;
+        if (!FULL) {
+          z0r = pa.z * cs + pa.w * sn;
+          z0i = pa.w * cs - pa.z * sn;
+        }
+        float2 zr = pk(z0r, z0r * pb.x - z0i * pb.y);
+        float2 zi = pk(z0i, z0r * pb.y + z0i * pb.x);
+        const float2 c2 = pk1(pb.z), s2 = pk1(pb.w), m2 = pk1(-pb.w);
 #pragma unroll
-          for (int q = 0; q < kMfF; ++q) {
-            const float kq = __fmaf_rn((float)q, k.dk, ks);
-            const float amp = pa.z * kq * sinc_acc(kq * pb.z) *
-                              sinc_acc(kq * pb.w);
-            acc[tt][q].x -= amp * ei;  // j amp e
-            acc[tt][q].y += amp * er;
-            const float nr = er * pb.x - ei * pb.y;
-            ei = er * pb.y + ei * pb.x;
-            er = nr;
+        for (int q = 0; q < kMfF / 2; ++q) {
+          if (FULL) {
+            float am[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const float kq = __fmaf_rn((float)(2 * q + h), k.dk, ks);
+              am[h] = pa.z * kq * sinc_acc(kq * s_pd[e].x) *
+                      sinc_acc(kq * s_pd[e].y);
+            }
+            const float2 av = pk(am[0], am[1]);
+            accr[tt][q] = sub2(accr[tt][q], mul2(av, zi));  // j amp e
+            acci[tt][q] = fma2(av, zr, acci[tt][q]);
+          } else {
+            accr[tt][q] = add2(accr[tt][q], zr);
+            acci[tt][q] = add2(acci[tt][q], zi);
           }
-        } else {
-          float zr = pa.z * er - pa.w * ei;
-          float zi = pa.z * ei + pa.w * er;
-#pragma unroll
-          for (int q = 0; q < kMfF; ++q) {
-            acc[tt][q].x += zr;
-            acc[tt][q].y += zi;
-            const float nr = zr * pb.x - zi * pb.y;
-            zi = zr * pb.y + zi * pb.x;
+          if (q + 1 < kMfF / 2) {
+            const float2 nr = fma2(zi, m2, mul2(zr, c2));
+            zi = fma2(zi, c2, mul2(zr, s2));
             zr = nr;
           }
         }
@@ -312,12 +359,18 @@ multifreq_split_kernel(MfArgs a, MfSplitConsts k) {
   }
   float2 *part = reinterpret_cast<float2 *>(a.part);
 #pragma unroll
-  for (int tt = 0; tt < kMfTB; ++tt) {
-    if (tt >= nt) break;
-    const size_t row = ((size_t)chunk * a.T + t_base + tt) * a.K;
+  for (int tt = 0; tt < kMfTB2; ++tt) {
+    const int t = half * kMfTB2 + tt;
+    if (t >= nt) break;
+    const size_t row = ((size_t)chunk * a.T + t_base + t) * a.K;
 #pragma unroll
-    for (int q = 0; q < kMfF; ++q)
-      if (kn + q < a.K) part[row + kn + q] = acc[tt][q];
+    for (int q = 0; q < kMfF / 2; ++q) {
+      if (kn + 2 * q < a.K)
+        part[row + kn + 2 * q] = make_float2(accr[tt][q].x, acci[tt][q].x);
+      if (kn + 2 * q + 1 < a.K)
+        part[row + kn + 2 * q + 1] =
+            make_float2(accr[tt][q].y, acci[tt][q].y);
+    }
   }
 }
 
@@ -356,14 +409,14 @@ multifreq_fp64_kernel(MfArgs a) {
   __syncthreads();
   const double dfq = a.bw / a.K;
   const double f1 = a.f0 - 0.5 * a.bw + 0.5 * dfq;
-  const int kn = blockIdx.z * kMfFBlock + tid * kMfF;
+  const int kn = blockIdx.z * kMfFBlock + tid * kMf64F;
   const double fs = f1 + kn * dfq;
   const double k0 = kTwoPi * a.f0 / a.c;
-  double2 acc[kMf64TB][kMfF];
+  double2 acc[kMf64TB][kMf64F];
 #pragma unroll
   for (int tt = 0; tt < kMf64TB; ++tt)
 #pragma unroll
-    for (int q = 0; q < kMfF; ++q) acc[tt][q] = make_double2(0.0, 0.0);
+    for (int q = 0; q < kMf64F; ++q) acc[tt][q] = make_double2(0.0, 0.0);
   for (int base = s_rng[0]; base < s_rng[1]; base += kMf64P) {
     for (int pr = tid; pr < kMf64TB * kMf64P; pr += blockDim.x) {
       const int tt = pr / kMf64P, i = base + pr % kMf64P;
@@ -411,7 +464,7 @@ multifreq_fp64_kernel(MfArgs a) {
         sincos(fmod(d[0] * fs, kTwoPi), &sn, &cs);
         double er = cs, ei = -sn;
         if (FULL) {
-          for (int q = 0; q < kMfF; ++q) {
+          for (int q = 0; q < kMf64F; ++q) {
             const double kq = kTwoPi * (fs + q * dfq) / a.c;
             const double amp = d[1] * kq * sinc_np(kq * d[2] / kPi) *
                                sinc_np(kq * d[3] / kPi);
@@ -424,7 +477,7 @@ multifreq_fp64_kernel(MfArgs a) {
         } else {
           // j amp exp(-j phase): (0 + j amp)(er + j ei)
           double zr = -d[2] * ei, zi = d[2] * er;
-          for (int q = 0; q < kMfF; ++q) {
+          for (int q = 0; q < kMf64F; ++q) {
             acc[tt][q].x += zr;
             acc[tt][q].y += zi;
             const double nr = zr * d[4] - zi * d[5];
@@ -441,7 +494,7 @@ multifreq_fp64_kernel(MfArgs a) {
   for (int tt = 0; tt < kMf64TB; ++tt) {
     if (tt >= nt) break;
     const size_t row = ((size_t)chunk * a.T + t_base + tt) * a.K;
-    for (int q = 0; q < kMfF; ++q)
+    for (int q = 0; q < kMf64F; ++q)
       if (kn + q < a.K) part[row + kn + q] = acc[tt][q];
   }
 }
@@ -454,69 +507,133 @@ constexpr int kSynTile = 256;
 // frequencies (drift <= 5e-7).
 constexpr int kSynAnchor = 8;
 
-template <bool F64>
+// FP64 form: one output sample per thread.
 __global__ void __launch_bounds__(kSynTile)
-multifreq_synth_kernel(int T, int K, int B, double f0, double bw,
-                       const double *H, const double *wbar,
-                       const double *twtt, double *y) {
+multifreq_synth64_kernel(int K, int B, double f0, double bw, const double *H,
+                         const double *wbar, const double *twtt, double *y) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int t = blockIdx.y;
   const int b = blockIdx.x * kSynTile + threadIdx.x;
   const double dfq = bw / K;
   const double f1 = f0 - 0.5 * bw + 0.5 * dfq;  // f_k - f0 = off + k dfq
   const double off = f1 - f0;
-  if (F64) {
-    double2 *g = reinterpret_cast<double2 *>(smem_raw);
-    for (int k = threadIdx.x; k < K; k += kSynTile)
-      g[k] = make_double2(wbar[k] * H[2 * ((size_t)t * K + k)],
-                          wbar[k] * H[2 * ((size_t)t * K + k) + 1]);
-    __syncthreads();
-    if (b >= B) return;
-    const double tau = twtt[b];
-    double sr, si;
-    const double cstep = dfq * tau;
-    sincospi(2.0 * (cstep - rint(cstep)), &si, &sr);
-    double yr = 0.0, yi = 0.0, er = 1.0, ei = 0.0;
-    for (int k = 0; k < K; ++k) {
-      if (k % kSynAnchor == 0) {
-        const double cyc = (off + k * dfq) * tau;
-        sincospi(2.0 * (cyc - rint(cyc)), &ei, &er);
-      }
-      yr += g[k].x * er - g[k].y * ei;
-      yi += g[k].x * ei + g[k].y * er;
-      const double nr = er * sr - ei * si;
-      ei = er * si + ei * sr;
-      er = nr;
+  double2 *g = reinterpret_cast<double2 *>(smem_raw);
+  for (int k = threadIdx.x; k < K; k += kSynTile)
+    g[k] = make_double2(wbar[k] * H[2 * ((size_t)t * K + k)],
+                        wbar[k] * H[2 * ((size_t)t * K + k) + 1]);
+  __syncthreads();
+  if (b >= B) return;
+  const double tau = twtt[b];
+  double sr, si;
+  const double cstep = dfq * tau;
+  sincospi(2.0 * (cstep - rint(cstep)), &si, &sr);
+  double yr = 0.0, yi = 0.0, er = 1.0, ei = 0.0;
+  for (int k = 0; k < K; ++k) {
+    if (k % kSynAnchor == 0) {
+      const double cyc = (off + k * dfq) * tau;
+      sincospi(2.0 * (cyc - rint(cyc)), &ei, &er);
     }
-    y[2 * ((size_t)t * B + b)] = yr;
-    y[2 * ((size_t)t * B + b) + 1] = yi;
-  } else {
-    float2 *g = reinterpret_cast<float2 *>(smem_raw);
-    for (int k = threadIdx.x; k < K; k += kSynTile)
-      g[k] = make_float2((float)(wbar[k] * H[2 * ((size_t)t * K + k)]),
-                         (float)(wbar[k] * H[2 * ((size_t)t * K + k) + 1]));
-    __syncthreads();
-    if (b >= B) return;
-    const double tau = twtt[b];
-    float sr, si;
-    const double cstep = dfq * tau;
-    sincospif((float)(2.0 * (cstep - rint(cstep))), &si, &sr);
-    Acc2 yr{0.0f, 0.0f}, yi{0.0f, 0.0f};
-    float er = 1.0f, ei = 0.0f;
-    for (int k = 0; k < K; ++k) {
-      if (k % kSynAnchor == 0) {
-        const double cyc = (off + k * dfq) * tau;
-        sincospif((float)(2.0 * (cyc - rint(cyc))), &ei, &er);
+    yr += g[k].x * er - g[k].y * ei;
+    yi += g[k].x * ei + g[k].y * er;
+    const double nr = er * sr - ei * si;
+    ei = er * si + ei * sr;
+    er = nr;
+  }
+  y[2 * ((size_t)t * B + b)] = yr;
+  y[2 * ((size_t)t * B + b) + 1] = yi;
+}
+
+// Split form: two output samples per thread, packed. An anchor's phase is a
+// double-float count of cycles (frequency offset, staged per anchor, times
+// the sample's delay) instead of a float64 one: at eight frequencies an
+// anchor the float64 pipe held the kernel (86% of its rate).
+constexpr int kSynThreads = 128;
+
+__device__ __forceinline__ void sincos_cycles(float fh, float fl, float th,
+                                              float tl, float &sn,
+                                              float &cs) {
+  float p, e;
+  two_prod(fh, th, p, e);
+  e = __fmaf_rn(fh, tl, __fmaf_rn(fl, th, e));
+  // quarter turns: 4 p = n + r, |r| <= 1/2 (the difference is exact)
+  const float t = rintf(4.0f * p);
+  const float r = __fmaf_rn(4.0f, p, -t) + 4.0f * e;
+  const float m = rintf(r);  // e may carry r past 1/2
+  const int q = (int)t + (int)m;
+  const float y = (r - m) * 1.57079632679489662f;
+  const float z = y * y;
+  const float s = __fmaf_rn(
+      __fmaf_rn(__fmaf_rn(-1.9515295891e-4f, z, 8.3321608736e-3f), z,
+                -1.6666654611e-1f) * z, y, y);
+  const float c = __fmaf_rn(
+      __fmaf_rn(__fmaf_rn(2.443315711809948e-5f, z, -1.388731625493765e-3f),
+                z, 4.166664568298827e-2f) * z, z, __fmaf_rn(-0.5f, z, 1.0f));
+  sn = (q & 1) ? c : s;
+  cs = (q & 1) ? s : c;
+  if (q & 2) sn = -sn;
+  if ((q + 1) & 2) cs = -cs;
+}
+
+__global__ void __launch_bounds__(kSynThreads)
+multifreq_synth_kernel(int K, int B, double f0, double bw, const double *H,
+                       const double *wbar, const double *twtt, double *y) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int t = blockIdx.y;
+  const int b0 = blockIdx.x * 2 * kSynThreads + threadIdx.x;
+  const int b1 = b0 + kSynThreads;
+  const double dfq = bw / K;
+  const double f1 = f0 - 0.5 * bw + 0.5 * dfq;  // f_k - f0 = off + k dfq
+  const double off = f1 - f0;
+  const int n_anchor = (K + kSynAnchor - 1) / kSynAnchor;
+  float2 *g = reinterpret_cast<float2 *>(smem_raw);
+  float2 *fo = g + K;  // anchor frequencies as double-floats
+  for (int k = threadIdx.x; k < K; k += kSynThreads)
+    g[k] = make_float2((float)(wbar[k] * H[2 * ((size_t)t * K + k)]),
+                       (float)(wbar[k] * H[2 * ((size_t)t * K + k) + 1]));
+  for (int k = threadIdx.x; k < n_anchor; k += kSynThreads) {
+    const df v = df_from_double(off + (double)(k * kSynAnchor) * dfq);
+    fo[k] = make_float2(v.hi, v.lo);
+  }
+  __syncthreads();
+  if (b0 >= B) return;
+  const df ta = df_from_double(twtt[b0]);
+  const df tb = df_from_double(twtt[min(b1, B - 1)]);
+  const df st = df_from_double(dfq);
+  float2 sr, si;
+  sincos_cycles(st.hi, st.lo, ta.hi, ta.lo, si.x, sr.x);
+  sincos_cycles(st.hi, st.lo, tb.hi, tb.lo, si.y, sr.y);
+  const float2 mi = pk(-si.x, -si.y);
+  const float2 zero = pk1(0.0f);
+  float2 yr = zero, yi = zero, cr = zero, ci = zero;
+  for (int k0 = 0; k0 < K; k0 += kSynAnchor) {
+    const float2 fk = fo[k0 / kSynAnchor];
+    float2 er, ei;
+    sincos_cycles(fk.x, fk.y, ta.hi, ta.lo, ei.x, er.x);
+    sincos_cycles(fk.x, fk.y, tb.hi, tb.lo, ei.y, er.y);
+    const int n = min(kSynAnchor, K - k0);
+#pragma unroll
+    for (int j = 0; j < kSynAnchor; ++j) {
+      if (j < n) {
+        const float2 gk = g[k0 + j];
+        const float2 gx = pk1(gk.x), gy = pk1(gk.y), my = pk1(-gk.y);
+        float2 e;
+        two_sum2(yr, fma2(gx, er, mul2(my, ei)), yr, e);
+        cr = add2(cr, e);
+        two_sum2(yi, fma2(gx, ei, mul2(gy, er)), yi, e);
+        ci = add2(ci, e);
+        const float2 nr = fma2(er, sr, mul2(ei, mi));
+        ei = fma2(er, si, mul2(ei, sr));
+        er = nr;
       }
-      const float2 gk = g[k];
-      acc2_add(yr, __fmaf_rn(gk.x, er, -gk.y * ei));
-      acc2_add(yi, __fmaf_rn(gk.x, ei, gk.y * er));
-      const float nr = er * sr - ei * si;
-      ei = er * si + ei * sr;
-      er = nr;
     }
-    y[2 * ((size_t)t * B + b)] = (double)yr.s + (double)yr.c;
-    y[2 * ((size_t)t * B + b) + 1] = (double)yi.s + (double)yi.c;
+  }
+  double *o = y + 2 * ((size_t)t * B + b0);
+  o[0] = (double)yr.x + (double)cr.x;
+  o[1] = (double)yi.x + (double)ci.x;
+  if (b1 < B) {
+    o = y + 2 * ((size_t)t * B + b1);
+    o[0] = (double)yr.y + (double)cr.y;
+    o[1] = (double)yi.y + (double)ci.y;
   }
 }
 
@@ -723,22 +840,27 @@ extern "C" int ss_multifreq_synth(const ss_multifreq_opts *o,
     return SS_ERR_UNSUPPORTED;
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  dim3 grid((n_twtt + kSynTile - 1) / kSynTile, n_traces);
   cudaError_t e;
   if (f64) {
-    e = cudaFuncSetAttribute(multifreq_synth_kernel<true>,
+    const dim3 grid((n_twtt + kSynTile - 1) / kSynTile, n_traces);
+    e = cudaFuncSetAttribute(multifreq_synth64_kernel,
                              cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem);
     if (e != cudaSuccess) return cuda_status(e, "synth smem");
-    multifreq_synth_kernel<true><<<grid, kSynTile, smem, st>>>(
-        n_traces, o->n_freq, n_twtt, o->f0, o->bandwidth, H, wbar, twtt, y);
+    multifreq_synth64_kernel<<<grid, kSynTile, smem, st>>>(
+        o->n_freq, n_twtt, o->f0, o->bandwidth, H, wbar, twtt, y);
   } else {
-    e = cudaFuncSetAttribute(multifreq_synth_kernel<false>,
+    const int per = 2 * kSynThreads;
+    const dim3 grid((n_twtt + per - 1) / per, n_traces);
+    // anchors besides (200 KB + 25 KB at most: within an SM's 227 KB)
+    const size_t sm = smem + (size_t)((o->n_freq + kSynAnchor - 1) /
+                                      kSynAnchor) * sizeof(float2);
+    e = cudaFuncSetAttribute(multifreq_synth_kernel,
                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
+                             (int)sm);
     if (e != cudaSuccess) return cuda_status(e, "synth smem");
-    multifreq_synth_kernel<false><<<grid, kSynTile, smem, st>>>(
-        n_traces, o->n_freq, n_twtt, o->f0, o->bandwidth, H, wbar, twtt, y);
+    multifreq_synth_kernel<<<grid, kSynThreads, sm, st>>>(
+        o->n_freq, n_twtt, o->f0, o->bandwidth, H, wbar, twtt, y);
   }
   return cuda_status(cudaGetLastError(), "multifreq synth launch");
 }
