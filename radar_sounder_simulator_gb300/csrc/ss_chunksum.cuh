@@ -11,6 +11,18 @@
 
 namespace ss {
 
+// A float as the same double, by its bits: the conversion instruction runs
+// on the float64 pipe, which held the reduce of small calls (one output bin
+// takes four). Zeros, subnormals, infinities and NaNs take the instruction.
+__device__ __forceinline__ double widen(float v) {
+  const unsigned int b = (unsigned int)__float_as_int(v);
+  const unsigned int ex = (b >> 23) & 0xffu;
+  if (ex - 1u >= 0xfeu) return (double)v;
+  const unsigned int hi = (b & 0x80000000u) | (((b >> 3) & 0x0fffffffu) +
+                                               0x38000000u);
+  return __hiloint2double((int)hi, (int)(b << 29));
+}
+
 template <typename P>
 struct ChunkSum;
 
@@ -24,7 +36,7 @@ struct ChunkSum<float> {
     l += e;
   }
   __device__ __forceinline__ double value() const {
-    return (double)h + (double)l;
+    return l == 0.0f ? widen(h) : widen(h) + widen(l);
   }
 };
 

@@ -15,6 +15,7 @@
 // streamed through shared memory in chunks of kTapChunk together with the
 // matching input window, so any pulse length works.
 #include "ss_df.cuh"
+#include "ss_f32x2.cuh"
 #include "ss_internal.cuh"
 
 namespace ss {
@@ -302,64 +303,98 @@ range_compress_fft_kernel(int B, int L, int N, int log_n, int center,
 //
 // Plan (once per pulse): twiddle table and pulse spectrum, 32 N bytes.
 // Apply: one CTA per (trace, lane) row, the row in shared memory as
-// float4 (re.hi, re.lo, im.hi, im.lo): 16 N bytes, two CTAs per SM at
-// N = 4096.
+// float4 (re.hi, im.hi, re.lo, im.lo): 16 N bytes, two CTAs per SM at
+// N = 4096. Real and imaginary parts run as packed pairs: the butterflies
+// were bound by the issue rate with the FMA pipe at 55%.
 // ---------------------------------------------------------------------
 constexpr int kDfThreads = 512;
 
+// A complex double-float as two pairs, high parts (re, im) and low parts:
+// every operation below runs re and im in one packed instruction.
 struct cdf {
-  df re, im;
+  float2 h, l;
 };
 
+__device__ __forceinline__ cdf c_unpack(float4 v) {
+  return cdf{make_float2(v.x, v.y), make_float2(v.z, v.w)};
+}
+
 __device__ __forceinline__ cdf c_ld(const float4 *x, int i) {
-  const float4 v = x[i];
-  return cdf{df{v.x, v.y}, df{v.z, v.w}};
+  return c_unpack(x[i]);
 }
 
 __device__ __forceinline__ cdf c_ldg(const float4 *x, int i) {
-  const float4 v = __ldg(x + i);
-  return cdf{df{v.x, v.y}, df{v.z, v.w}};
+  return c_unpack(__ldg(x + i));
 }
 
 __device__ __forceinline__ void c_st(float4 *x, int i, const cdf &a) {
-  x[i] = make_float4(a.re.hi, a.re.lo, a.im.hi, a.im.lo);
+  x[i] = make_float4(a.h.x, a.h.y, a.l.x, a.l.y);
 }
 
+// Dekker's sum of |a| >= |b|, renormalising a pair of double-floats.
+__device__ __forceinline__ cdf c_norm(float2 h, float2 l) {
+  cdf r;
+  r.h = add2(h, l);
+  r.l = sub2(l, sub2(r.h, h));
+  return r;
+}
+
+// Sums stay unnormalised: their low part carries a few ulp of the high one
+// until the next product renormalises it (six stages at most), which costs
+// the products' dropped low x low term two or three bits of 2^-48.
 __device__ __forceinline__ cdf c_add(const cdf &a, const cdf &b) {
-  return cdf{df_add(a.re, b.re), df_add(a.im, b.im)};
+  cdf r;
+  float2 e;
+  two_sum2(a.h, b.h, r.h, e);
+  r.l = add2(e, add2(a.l, b.l));
+  return r;
 }
 
 __device__ __forceinline__ cdf c_sub(const cdf &a, const cdf &b) {
-  return cdf{df_sub(a.re, b.re), df_sub(a.im, b.im)};
+  // a + (-b): s + e == a.h - b.h exactly
+  const float2 s = sub2(a.h, b.h);
+  const float2 bb = sub2(a.h, s);  // the part of b.h that s took
+  const float2 e = add2(sub2(a.h, add2(s, bb)), sub2(bb, b.h));
+  return cdf{s, add2(e, sub2(a.l, b.l))};
 }
 
-// a b + c d: both leading products exact (FMA two-product) and summed by
-// a two-sum, the cross terms added to the low part
-__device__ __forceinline__ df df_dot2(df a, df b, df c, df d) {
-  float p1, e1, p2, e2, s, e3;
-  two_prod(a.hi, b.hi, p1, e1);
-  two_prod(c.hi, d.hi, p2, e2);
-  two_sum(p1, p2, s, e3);
-  float lo = (e1 + e2) + e3;
-  lo = __fmaf_rn(a.hi, b.lo, __fmaf_rn(a.lo, b.hi, lo));
-  lo = __fmaf_rn(c.hi, d.lo, __fmaf_rn(c.lo, d.hi, lo));
-  return df_make(s, lo);
+// a w: both leading products of each component exact (FMA two-product) and
+// summed by a two-sum, the cross terms added to the low part. wp = w, wq =
+// i w, so that a w = a.re wp + a.im wq.
+__device__ __forceinline__ cdf c_mul2(const cdf &a, const cdf &wp,
+                                      const cdf &wq) {
+  const float2 rh = pk1(a.h.x), ih = pk1(a.h.y);
+  const float2 rl = pk1(a.l.x), il = pk1(a.l.y);
+  const float2 p1 = mul2(rh, wp.h), p2 = mul2(ih, wq.h);
+  const float2 n1 = pk(-p1.x, -p1.y), n2 = pk(-p2.x, -p2.y);
+  const float2 e1 = fma2(rh, wp.h, n1), e2 = fma2(ih, wq.h, n2);
+  float2 s, e3;
+  two_sum2(p1, p2, s, e3);
+  float2 lo = add2(add2(e1, e2), e3);
+  lo = fma2(rh, wp.l, fma2(rl, wp.h, lo));
+  lo = fma2(ih, wq.l, fma2(il, wq.h, lo));
+  return c_norm(s, lo);
+}
+
+// i w and, for the inverse transform, conj(w) and i conj(w).
+__device__ __forceinline__ cdf c_iw(const cdf &w) {
+  return cdf{pk(-w.h.y, w.h.x), pk(-w.l.y, w.l.x)};
+}
+
+__device__ __forceinline__ cdf c_conj(const cdf &a) {
+  return cdf{pk(a.h.x, -a.h.y), pk(a.l.x, -a.l.y)};
 }
 
 __device__ __forceinline__ cdf c_mul(const cdf &a, const cdf &w) {
-  return cdf{df_dot2(a.re, w.re, df_neg(a.im), w.im),
-             df_dot2(a.re, w.im, a.im, w.re)};
+  return c_mul2(a, w, c_iw(w));
 }
 
-__device__ __forceinline__ cdf c_conj(cdf a) {
-  a.im = df_neg(a.im);
-  return a;
-}
-
-// Forward transform in place, natural order in, digit-reversed out.
+// Forward transform in place, natural order in, digit-reversed out; `stop`
+// leaves out the innermost stage (quarter lengths below 2^stop, and with it
+// the radix-2 stage), which df_fft_middle runs.
 __device__ void df_fft_forward(float4 *x, int N, int lg,
-                               const float4 *__restrict__ tw) {
-  for (int lq = lg - 2; lq >= 0; lq -= 2) {
+                               const float4 *__restrict__ tw, int stop = 0) {
+  for (int lq = lg - 2; lq >= stop; lq -= 2) {
     const int q = 1 << lq;
     const float4 *T = tw + (N - 4 * q);
     for (int b = threadIdx.x; b < (N >> 2); b += blockDim.x) {
@@ -369,7 +404,7 @@ __device__ void df_fft_forward(float4 *x, int N, int lg,
                 a2 = c_ld(x, base + 2 * q), a3 = c_ld(x, base + 3 * q);
       const cdf b0 = c_add(a0, a2), b1 = c_sub(a0, a2), b2 = c_add(a1, a3),
                 b3 = c_sub(a1, a3);
-      const cdf mib3{b3.im, df_neg(b3.re)};  // -i b3
+      const cdf mib3{pk(b3.h.y, -b3.h.x), pk(b3.l.y, -b3.l.x)};  // -i b3
       c_st(x, base, c_add(b0, b2));
       c_st(x, base + q, c_mul(c_add(b1, mib3), c_ldg(T, 3 * j)));
       c_st(x, base + 2 * q, c_mul(c_sub(b0, b2), c_ldg(T, 3 * j + 1)));
@@ -377,7 +412,7 @@ __device__ void df_fft_forward(float4 *x, int N, int lg,
     }
     __syncthreads();
   }
-  if (lg & 1) {
+  if ((lg & 1) && !stop) {
     for (int b = threadIdx.x; b < (N >> 1); b += blockDim.x) {
       const cdf a0 = c_ld(x, 2 * b), a1 = c_ld(x, 2 * b + 1);
       c_st(x, 2 * b, c_add(a0, a1));
@@ -387,18 +422,47 @@ __device__ void df_fft_forward(float4 *x, int N, int lg,
   }
 }
 
-// Inverse transform in place (unscaled), digit-reversed in, natural out.
-__device__ void df_fft_inverse(float4 *x, int N, int lg,
-                               const float4 *__restrict__ tw) {
+// The innermost stage both ways around the product with the pulse spectrum,
+// in registers: blocks of length 4 (log2 N even) or 2 (odd), whose twiddles
+// are all 1, so their products and two passes over shared memory go.
+__device__ void df_fft_middle(float4 *x, int N, int lg,
+                              const float4 *__restrict__ spec) {
   if (lg & 1) {
     for (int b = threadIdx.x; b < (N >> 1); b += blockDim.x) {
       const cdf a0 = c_ld(x, 2 * b), a1 = c_ld(x, 2 * b + 1);
-      c_st(x, 2 * b, c_add(a0, a1));
-      c_st(x, 2 * b + 1, c_sub(a0, a1));
+      const cdf u = c_mul(c_add(a0, a1), c_ldg(spec, 2 * b));
+      const cdf v = c_mul(c_sub(a0, a1), c_ldg(spec, 2 * b + 1));
+      c_st(x, 2 * b, c_add(u, v));
+      c_st(x, 2 * b + 1, c_sub(u, v));
     }
-    __syncthreads();
+  } else {
+    for (int b = threadIdx.x; b < (N >> 2); b += blockDim.x) {
+      cdf c[4];
+      {
+        const cdf a0 = c_ld(x, 4 * b), a1 = c_ld(x, 4 * b + 1),
+                  a2 = c_ld(x, 4 * b + 2), a3 = c_ld(x, 4 * b + 3);
+        const cdf b0 = c_add(a0, a2), b1 = c_sub(a0, a2),
+                  b2 = c_add(a1, a3), ib3 = c_iw(c_sub(a1, a3));
+        c[0] = c_mul(c_add(b0, b2), c_ldg(spec, 4 * b));
+        c[1] = c_mul(c_sub(b1, ib3), c_ldg(spec, 4 * b + 1));
+        c[2] = c_mul(c_sub(b0, b2), c_ldg(spec, 4 * b + 2));
+        c[3] = c_mul(c_add(b1, ib3), c_ldg(spec, 4 * b + 3));
+      }
+      const cdf d0 = c_add(c[0], c[2]), d1 = c_sub(c[0], c[2]),
+                d2 = c_add(c[1], c[3]), id3 = c_iw(c_sub(c[1], c[3]));
+      c_st(x, 4 * b, c_add(d0, d2));
+      c_st(x, 4 * b + 1, c_add(d1, id3));
+      c_st(x, 4 * b + 2, c_sub(d0, d2));
+      c_st(x, 4 * b + 3, c_sub(d1, id3));
+    }
   }
-  for (int lq = lg & 1; lq <= lg - 2; lq += 2) {
+  __syncthreads();
+}
+
+// Inverse transform (unscaled) of what df_fft_middle leaves, natural out.
+__device__ void df_fft_inverse(float4 *x, int N, int lg,
+                               const float4 *__restrict__ tw) {
+  for (int lq = (lg & 1) ? 1 : 2; lq <= lg - 2; lq += 2) {
     const int q = 1 << lq;
     const float4 *T = tw + (N - 4 * q);
     for (int b = threadIdx.x; b < (N >> 2); b += blockDim.x) {
@@ -410,7 +474,7 @@ __device__ void df_fft_inverse(float4 *x, int N, int lg,
       const cdf c3 = c_mul(c_ld(x, base + 3 * q), c_conj(c_ldg(T, 3 * j + 2)));
       const cdf d0 = c_add(c0, c2), d1 = c_sub(c0, c2), d2 = c_add(c1, c3),
                 d3 = c_sub(c1, c3);
-      const cdf id3{df_neg(d3.im), d3.re};  // +i d3
+      const cdf id3 = c_iw(d3);  // +i d3
       c_st(x, base, c_add(d0, d2));
       c_st(x, base + q, c_add(d1, id3));
       c_st(x, base + 2 * q, c_sub(d0, d2));
@@ -433,7 +497,7 @@ __global__ void df_twiddle_kernel(int N, int lg, float4 *tw) {
         double s, c;
         sincospi(-2.0 * (double)t / (double)N, &s, &c);
         const df dc = df_from_double(c), ds = df_from_double(s);
-        v = make_float4(dc.hi, dc.lo, ds.hi, ds.lo);
+        v = make_float4(dc.hi, ds.hi, dc.lo, ds.lo);
       }
     }
     tw[e] = v;
@@ -452,7 +516,7 @@ df_pulse_kernel(int N, int lg, int n_taps, int power, const double *taps,
       re = df_from_double(power ? taps[i] : taps[2 * i]);
       if (!power) im = df_from_double(taps[2 * i + 1]);
     }
-    c_st(x, i, cdf{re, im});
+    x[i] = make_float4(re.hi, im.hi, re.lo, im.lo);
   }
   __syncthreads();
   df_fft_forward(x, N, lg, plan + N);
@@ -487,13 +551,11 @@ range_compress_df_kernel(int B, int L, int N, int lg, int center,
         vi = f.y;
       }
     }
-    x[i] = make_float4(vr, 0.0f, vi, 0.0f);
+    x[i] = make_float4(vr, vi, 0.0f, 0.0f);
   }
   __syncthreads();
-  df_fft_forward(x, N, lg, plan + N);
-  for (int i = threadIdx.x; i < N; i += blockDim.x)
-    c_st(x, i, c_mul(c_ld(x, i), c_ldg(plan, i)));
-  __syncthreads();
+  df_fft_forward(x, N, lg, plan + N, (lg & 1) ? 1 : 2);
+  df_fft_middle(x, N, lg, plan);
   df_fft_inverse(x, N, lg, plan + N);
   const float inv = 1.0f / (float)N;  // a power of two: exact
   for (int i = threadIdx.x; i < B; i += blockDim.x) {
@@ -501,10 +563,10 @@ range_compress_df_kernel(int B, int L, int N, int lg, int center,
     const size_t e = ((size_t)t * B + i) * L + l;
     // hi + lo rounds the double-float once to float32
     if (POWER)
-      static_cast<float *>(out)[e] = fmaxf((y.x + y.y) * inv, 0.0f);
+      static_cast<float *>(out)[e] = fmaxf((y.x + y.z) * inv, 0.0f);
     else
       static_cast<float2 *>(out)[e] =
-          make_float2((y.x + y.y) * inv, (y.z + y.w) * inv);
+          make_float2((y.x + y.z) * inv, (y.y + y.w) * inv);
   }
 }
 
