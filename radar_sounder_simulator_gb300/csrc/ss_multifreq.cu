@@ -53,10 +53,19 @@ struct MfArgs {
 // traces, each thread 16 frequencies as two interleaved chains of 8 -- one
 // packed instruction advances both -- so the carrier phase's head (product,
 // reduction, sine and cosine) is paid once per 16 and a chain is as long as
-// the 8 frequencies a float32 step may drift over.
+// the 8 frequencies a float32 step may drift over. A CTA has as many threads
+// as its share of the band needs (768 frequencies: 2 x 48; at a fixed 128 a
+// quarter of the lanes idled, 0.39 -> 0.31 ms at 96 x 128 facets x 100
+// traces).
 constexpr int kMfThreads = 128, kMfF = 16, kMfTB = 4, kMfP = 32;
-constexpr int kMfHalf = kMfThreads / 2, kMfTB2 = kMfTB / 2;
-constexpr int kMfFBlock = kMfHalf * kMfF;
+constexpr int kMfTB2 = kMfTB / 2;
+constexpr int kMfFBlock = kMfThreads / 2 * kMfF;
+
+// Threads of half a CTA for K frequencies cut into equal blocks.
+static int mf_half(int K) {
+  const int blocks = (K + kMfFBlock - 1) / kMfFBlock;
+  return ((K + blocks - 1) / blocks + kMfF - 1) / kMfF;
+}
 // FP64 form: 128 threads x 8 frequencies
 constexpr int kMf64F = 8;
 // FP64 form: 2 traces per CTA, tiles of 64 facets
@@ -187,8 +196,8 @@ multifreq_split_kernel(MfArgs a, MfSplitConsts k) {
   __syncthreads();
 
   // this thread's first frequency index and its frequency / wavenumber
-  const int half = tid / kMfHalf;
-  const int kn = blockIdx.z * kMfFBlock + (tid % kMfHalf) * kMfF;
+  const int n_half = blockDim.x / 2, half = tid / n_half;
+  const int kn = (blockIdx.z * n_half + tid - half * n_half) * kMfF;
   float fsh, fsl;
   {
     float p, e;
@@ -208,9 +217,10 @@ multifreq_split_kernel(MfArgs a, MfSplitConsts k) {
       accr[tt][q] = acci[tt][q] = make_float2(0.0f, 0.0f);
 
   for (int base = s_rng[0]; base < s_rng[1]; base += kMfP) {
-    // --- phase A: one (trace, facet) pair per thread ---
-    {
-      const int tt = tid / kMfP, i = base + tid % kMfP;
+    // --- phase A: the tile's (trace, facet) pairs ---
+    __syncthreads();
+    for (int e0 = tid; e0 < kMfTB * kMfP; e0 += blockDim.x) {
+      const int tt = e0 / kMfP, i = base + e0 % kMfP;
       float4 pa = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       float4 pb = make_float4(1.0f, 0.0f, 1.0f, 0.0f);
       float2 pd = make_float2(0.0f, 0.0f);
@@ -298,13 +308,12 @@ multifreq_split_kernel(MfArgs a, MfSplitConsts k) {
           pa = make_float4(Rh, Rl, -ci, cr);
         }
       }
-      __syncthreads();
-      s_pa[tid] = pa;
-      s_pb[tid] = pb;
-      if (FULL) s_pd[tid] = pd;
-      __syncthreads();
+      s_pa[e0] = pa;
+      s_pb[e0] = pb;
+      if (FULL) s_pd[e0] = pd;
     }
-    if (kn >= a.K) continue;  // whole warps past the band's end
+    __syncthreads();
+    if (kn >= a.K) continue;  // past the band's end
     // --- phase B: every thread, its traces' pairs, its frequencies ---
 #pragma unroll
     for (int tt = 0; tt < kMfTB2; ++tt) {
@@ -758,6 +767,7 @@ extern "C" int ss_multifreq_response(const ss_multifreq_opts *o,
   cudaError_t e = cudaMemsetAsync(part_drop, 0, drop, st);
   if (e != cudaSuccess) return cuda_status(e, "multifreq scratch clear");
   const int fblk = (a.K + kMfFBlock - 1) / kMfFBlock;
+  const int threads = 2 * mf_half(a.K);  // split form
   dim3 grid(p.n_chunks, p.n_groups, fblk);
   if (f64) {
     if (o->freeze_amplitudes)
@@ -790,24 +800,24 @@ extern "C" int ss_multifreq_response(const ss_multifreq_opts *o,
     const size_t smem = rk ? (size_t)(a.n_terms + 1) * sizeof(float) : 0;
     if (!o->freeze_amplitudes) {
       multifreq_split_kernel<true, SS_ROUGH_NONE>
-          <<<grid, kMfThreads, smem, st>>>(a, k);
+          <<<grid, threads, smem, st>>>(a, k);
     } else {
       switch (rk) {
         case SS_ROUGH_NONE:
           multifreq_split_kernel<false, SS_ROUGH_NONE>
-              <<<grid, kMfThreads, smem, st>>>(a, k);
+              <<<grid, threads, smem, st>>>(a, k);
           break;
         case SS_ROUGH_GAUSS_FULL:
           multifreq_split_kernel<false, SS_ROUGH_GAUSS_FULL>
-              <<<grid, kMfThreads, smem, st>>>(a, k);
+              <<<grid, threads, smem, st>>>(a, k);
           break;
         case SS_ROUGH_GAUSS_AREA:
           multifreq_split_kernel<false, SS_ROUGH_GAUSS_AREA>
-              <<<grid, kMfThreads, smem, st>>>(a, k);
+              <<<grid, threads, smem, st>>>(a, k);
           break;
         default:
           multifreq_split_kernel<false, SS_ROUGH_EXP_AREA>
-              <<<grid, kMfThreads, smem, st>>>(a, k);
+              <<<grid, threads, smem, st>>>(a, k);
           break;
       }
     }
