@@ -237,10 +237,10 @@ static int refracted_plan(const ss_refracted_opts *o, int T, int N, Plan *p) {
   } else {
     // resident CTAs per SM of the split kernel that runs: two 512-thread
     // CTAs (64 registers) for the sequential chain and joint solves through
-    // up to two interfaces, one (~128 registers) through three or more
+    // one interface, one (~128 registers) through two or more
     const int max_chunks = (int)std::max<long>(1, window / 256);
     const long slots = (long)sm_count() *
-                       (!o->joint || o->n_crossed <= 2 ? 2 : 1);
+                       (!o->joint || o->n_crossed <= 1 ? 2 : 1);
     p->n_groups = (T + tb - 1) / tb;
     p->n_chunks = wave_chunks(slots, p->n_groups, max_chunks, 4, 12);
   }

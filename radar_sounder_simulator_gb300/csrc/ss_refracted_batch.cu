@@ -69,11 +69,13 @@ struct RefBatchLayout {
   size_t table_off = 256, mask_off = 0, bytes = 0, smem = 0;
   long long n_items = 0, n_out = 0, n_words = 0;
   int path_class = 0, rough_kind = 0, plain = 1;
+  bool short_form = false;
 };
 
-// Path class of a batch whose sequential jobs all cross one interface
-// (kOneNI kernels); 0 is the general sequential chain, 1-4 the joint solve.
-constexpr int kBatchOne = 5;
+// The kernels of a batch: `plain` (bit 0) for the plain instantiation, bit 1
+// when every job takes the short form of its path class (single crossing for
+// the sequential class, lean joint solve).
+constexpr int kBatchPlain = 1, kBatchShort = 2;
 
 static bool job_plain(const RefArgs &a) {
   return a.rough_kind == SS_ROUGH_NONE && a.pat_kind == SS_PAT_ISOTROPIC &&
@@ -102,7 +104,7 @@ static int ref_batch_layout(const ss_refracted_job *jobs, int n_jobs,
   }
   L.jobs.assign(n_jobs, RefBatchJob{});
   double total_pairs = 0.0;
-  bool all_one = true;
+  bool all_one = true, all_lean = true;
   std::vector<long long> window(n_jobs);
   for (int j = 0; j < n_jobs; ++j) {
     const ss_refracted_job &q = jobs[j];
@@ -137,6 +139,7 @@ static int ref_batch_layout(const ss_refracted_job *jobs, int n_jobs,
     }
     L.plain = L.plain && job_plain(a);
     all_one = all_one && one_crossing(a);
+    all_lean = all_lean && lean_joint(a);
     const size_t per_trace = (size_t)a.n_seg * sizeof(float2);
     a.tb = (int)std::min<size_t>(
         std::max<size_t>(1, std::min<size_t>(96 * 1024 / per_trace, max_tb)),
@@ -145,7 +148,7 @@ static int ref_batch_layout(const ss_refracted_job *jobs, int n_jobs,
     window[j] = std::min<long long>((long long)a.n_win * a.bs, a.N);
     total_pairs += (double)a.T * window[j];
   }
-  if (all_one) L.path_class = kBatchOne;
+  L.short_form = all_one || all_lean;
   const double per_item =
       std::max(1.0, total_pairs / ((double)ips * sm_count()));
   // The queue serves the costliest jobs first (longest-processing-time
@@ -212,15 +215,20 @@ static int ref_batch_layout(const ss_refracted_job *jobs, int n_jobs,
   return SS_OK;
 }
 
-static int ref_batch_occupancy_class(int cls, int rough, bool plain,
-                                     size_t smem) {
-  switch (cls) {
-    case 0: return refracted_batch_occupancy_ni0(rough, plain, smem);
-    case 1: return refracted_batch_occupancy_ni1(rough, plain, smem);
-    case 2: return refracted_batch_occupancy_ni2(rough, plain, smem);
-    case 3: return refracted_batch_occupancy_ni3(rough, plain, smem);
-    case kBatchOne: return refracted_batch_occupancy_nione(rough, plain, smem);
-    default: return refracted_batch_occupancy_ni4(rough, plain, smem);
+static int ref_batch_occupancy_class(const RefBatchLayout &L) {
+  const int r = L.rough_kind;
+  const bool p = L.plain != 0;
+  switch (L.path_class + (L.short_form ? 5 : 0)) {
+    case 0: return refracted_batch_occupancy_ni0(r, p, L.smem);
+    case 1: return refracted_batch_occupancy_ni1(r, p, L.smem);
+    case 2: return refracted_batch_occupancy_ni2(r, p, L.smem);
+    case 3: return refracted_batch_occupancy_ni3(r, p, L.smem);
+    case 4: return refracted_batch_occupancy_ni4(r, p, L.smem);
+    case 5: return refracted_batch_occupancy_nione(r, p, L.smem);
+    case 6: return refracted_batch_occupancy_nilean1(r, p, L.smem);
+    case 7: return refracted_batch_occupancy_nilean2(r, p, L.smem);
+    case 8: return refracted_batch_occupancy_nilean3(r, p, L.smem);
+    default: return refracted_batch_occupancy_nilean4(r, p, L.smem);
   }
 }
 
@@ -259,8 +267,7 @@ extern "C" int ss_refracted_batch_prepare(const ss_refracted_job *jobs,
     J.a.defer_mask = reinterpret_cast<uint32_t *>(
         base + reinterpret_cast<size_t>(J.a.defer_mask));
   }
-  int per_sm = ref_batch_occupancy_class(L.path_class, L.rough_kind,
-                                         L.plain != 0, L.smem);
+  int per_sm = ref_batch_occupancy_class(L);
   if (per_sm <= 0) {
     set_error("batched refracted kernel does not fit on an SM with this "
               "shared memory");
@@ -276,7 +283,8 @@ extern "C" int ss_refracted_batch_prepare(const ss_refracted_job *jobs,
   info->n_jobs = n_jobs;
   info->path_class = L.path_class;
   info->rough_kind = L.rough_kind;
-  info->plain = L.plain;
+  info->plain = (L.plain ? kBatchPlain : 0) |
+                (L.short_form ? kBatchShort : 0);
   info->ctas = per_sm * sm_count();
   info->n_items = L.n_items;
   info->n_out = L.n_out;
@@ -306,19 +314,23 @@ extern "C" int ss_refracted_batch_run(const ss_refracted_batch_info *info,
                       (size_t)info->n_words * sizeof(uint32_t), st);
   if (e != cudaSuccess) return cuda_status(e, "batch mask clear");
   int s;
-  const bool plain = info->plain != 0;
+  const bool plain = (info->plain & kBatchPlain) != 0;
 #define SS_RB(N)                                                              \
   refracted_batch_launch_ni##N(jobs, info->n_jobs, info->n_items,           \
                                info->n_words, counter, info->rough_kind,     \
                                plain, info->ctas, info->smem,                \
                                info->fix_smem, st)
-  switch (info->path_class) {
+  switch (info->path_class + ((info->plain & kBatchShort) ? 5 : 0)) {
     case 0: s = SS_RB(0); break;
     case 1: s = SS_RB(1); break;
     case 2: s = SS_RB(2); break;
     case 3: s = SS_RB(3); break;
-    case kBatchOne: s = SS_RB(one); break;
-    default: s = SS_RB(4); break;
+    case 4: s = SS_RB(4); break;
+    case 5: s = SS_RB(one); break;
+    case 6: s = SS_RB(lean1); break;
+    case 7: s = SS_RB(lean2); break;
+    case 8: s = SS_RB(lean3); break;
+    default: s = SS_RB(lean4); break;
   }
 #undef SS_RB
   if (s) return s;

@@ -148,13 +148,16 @@ __device__ __forceinline__ void one_facet(const OnePlane &M, const float *q,
 // float64 (six scenes of 300-2500 m depth, 3-25 km altitude, 25 and 50 m
 // cells, a million pairs each) errs by at most 6.5e-7 of one cell plus the
 // offset; the band is over four times that.
+// Down a chain of interfaces the error grows slowly (1.0e-6 at the third):
+// `scale` widens the band there.
 constexpr float kCellAbs = 5e-6f, kCellRel = 3e-6f;
 
-// Cell of the mean-plane crossing of p - q = P; false when a coordinate is
-// within the guard band of a rounding boundary.
+// Cell of the mean-plane crossing of the ray from q + P to q, and that
+// crossing from q (v, which may be P); false when a coordinate is within the
+// guard band of a rounding boundary.
 __device__ __forceinline__ bool one_cell(const OnePlane &M, const OneFacet &f,
                                          const float *P, int ny, int nx,
-                                         int &cell) {
+                                         float scale, int &cell, float *v) {
   const float vn = dot3f(P[0], P[1], P[2], M.mn[0], M.mn[1], M.mn[2]);
   const float wx = __fmaf_rn(-vn, M.mn[0], P[0]);
   const float wy = __fmaf_rn(-vn, M.mn[1], P[1]);
@@ -170,9 +173,13 @@ __device__ __forceinline__ bool one_cell(const OnePlane &M, const OneFacet &f,
   const float row = fminf(fmaxf(f.ri[0] + kr, 0.0f), (float)(ny - 1));
   const float col = fminf(fmaxf(f.ri[1] + kc, 0.0f), (float)(nx - 1));
   cell = (int)row * nx + (int)col;
-  return fmaxf(__fmaf_rn(kCellRel, fabsf(fr), fabsf(fr - kr)),
-               __fmaf_rn(kCellRel, fabsf(fc), fabsf(fc - kc))) <
-         0.5f - kCellAbs;
+  v[0] = __fmaf_rn(g, wx, f.b * M.mn[0]);
+  v[1] = __fmaf_rn(g, wy, f.b * M.mn[1]);
+  v[2] = __fmaf_rn(g, wz, f.b * M.mn[2]);
+  const float rel = kCellRel * scale;
+  return fmaxf(__fmaf_rn(rel, fabsf(fr), fabsf(fr - kr)),
+               __fmaf_rn(rel, fabsf(fc), fabsf(fc - kc))) <
+         0.5f - kCellAbs * scale;
 }
 
 // |v| of a vector of floats taken as exact, as a double-float; `inv` its
@@ -221,6 +228,48 @@ struct PairGeo {
   bool valid;
 };
 
+// Plane point o and stored normal t of a table cell.
+__device__ __forceinline__ void load_plane(int vec,
+                                           const float *__restrict__ table,
+                                           int cell, float *o, float *t) {
+  const float *g = table + (size_t)cell * 6;
+  if (vec) {
+    const float2 u0 = __ldg(reinterpret_cast<const float2 *>(g)),
+                 u1 = __ldg(reinterpret_cast<const float2 *>(g) + 1),
+                 u2 = __ldg(reinterpret_cast<const float2 *>(g) + 2);
+    o[0] = u0.x; o[1] = u0.y; o[2] = u1.x;
+    t[0] = u1.y; t[1] = u2.x; t[2] = u2.y;
+  } else {
+    for (int j = 0; j < 3; ++j) {
+      o[j] = __ldg(g + j);
+      t[j] = __ldg(g + 3 + j);
+    }
+  }
+}
+
+// t . (y - (o - q)) from exact differences and products: the height of the
+// crossing q + y over the plane of normal t through o, to float32 precision
+// of the height itself.
+__device__ __forceinline__ float plane_offset(const float *y, const float *o,
+                                              const float *q,
+                                              const float *t) {
+  float d[3], dl[3], p0, e0, p1, e1, p2, e2, sh, f1, f2;
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    float oh, ol;
+    two_sum(o[j], -q[j], oh, ol);
+    two_sum(y[j], -oh, d[j], dl[j]);
+    dl[j] -= ol;
+  }
+  two_prod(d[0], t[0], p0, e0);
+  two_prod(d[1], t[1], p1, e1);
+  two_prod(d[2], t[2], p2, e2);
+  two_sum(p0, p1, sh, f1);
+  two_sum(sh, p2, sh, f2);
+  return sh + ((f1 + f2) + (e0 + e1 + e2) +
+               dot3f(dl[0], dl[1], dl[2], t[0], t[1], t[2]));
+}
+
 // Scalars of the one-crossing pair.
 struct OneLegs {
   float n1, n1l, n2, n2l, i1, i2;  // indices (double-float), reciprocals
@@ -245,30 +294,15 @@ __device__ __forceinline__ void one_path(const OnePlane &M, const OneLegs &k,
                                          int cell, const float *q,
                                          const float *Ph, const float *Pl,
                                          float tol, PairGeo &G) {
-  const float *g = table + (size_t)cell * 6;
   float o[3], t[3];
-  if (M.vec) {
-    const float2 u0 = __ldg(reinterpret_cast<const float2 *>(g)),
-                 u1 = __ldg(reinterpret_cast<const float2 *>(g) + 1),
-                 u2 = __ldg(reinterpret_cast<const float2 *>(g) + 2);
-    o[0] = u0.x; o[1] = u0.y; o[2] = u1.x;
-    t[0] = u1.y; t[1] = u2.x; t[2] = u2.y;
-  } else {
-    for (int j = 0; j < 3; ++j) {
-      o[j] = __ldg(g + j);
-      t[j] = __ldg(g + 3 + j);
-    }
-  }
+  load_plane(M.vec, table, cell, o, t);
   // unit normal to float32 rounding (one Newton step on the seed)
   const float nn = dot3f(t[0], t[1], t[2], t[0], t[1], t[2]);
   float in = rsq_n(nn);
   in = in * __fmaf_rn(-0.5f * nn * in, in, 1.5f);
   const float n[3] = {t[0] * in, t[1] * in, t[2] * in};
-  // plane point from q, exactly: hi oh, lo ol
-  float oh[3], ol[3];
-#pragma unroll
-  for (int j = 0; j < 3; ++j) two_sum(o[j], -q[j], oh[j], ol[j]);
-  const float b = dot3f(oh[0], oh[1], oh[2], n[0], n[1], n[2]);
+  const float b = dot3f(o[0] - q[0], o[1] - q[1], o[2] - q[2], n[0], n[1],
+                        n[2]);
   const float vn = dot3f(Ph[0], Ph[1], Ph[2], n[0], n[1], n[2]);
   const float a = vn - b;
   float w[3];
@@ -295,19 +329,7 @@ __device__ __forceinline__ void one_path(const OnePlane &M, const OneLegs &k,
   // rounding (up to ~1e-4 m), which the optical path takes at first order;
   // its height over that plane towards the upper point, from exact
   // products, times the legs' index-weighted cosines puts it back.
-  float d[3], dl[3], p0, e0, p1, e1, p2, e2, sh, f1, f2;
-#pragma unroll
-  for (int j = 0; j < 3; ++j) {
-    two_sum(y[j], -oh[j], d[j], dl[j]);
-    dl[j] -= ol[j];
-  }
-  two_prod(d[0], t[0], p0, e0);
-  two_prod(d[1], t[1], p1, e1);
-  two_prod(d[2], t[2], p2, e2);
-  two_sum(p0, p1, sh, f1);
-  two_sum(sh, p2, sh, f2);
-  float hp = sh + ((f1 + f2) + (e0 + e1 + e2) +
-                   dot3f(dl[0], dl[1], dl[2], t[0], t[1], t[2]));
+  float hp = plane_offset(y, o, q, t);
   hp = a >= 0.0f ? hp : -hp;
   const float nc1 = k.n1 * c1, nc2 = k.n2 * c2;
   // optical path n1 s1 + n2 s2 + hp (n1 c1 - n2 c2)

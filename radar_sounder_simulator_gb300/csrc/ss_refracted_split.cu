@@ -37,9 +37,11 @@ RefSplitConsts split_consts(const RefArgs &a) {
   const double og = (!a.joint && a.ni > 1) ? kOplGuardChain : 0.0;
   k.bin_guard = (float)std::max((double)kBinGuard, og * 2.0 / (a.c * a.dt));
   k.gamma = (float)a.gamma;
-  {
-    OnePlane &O = k.one;
-    const ss_interface &I = a.ifc[0];
+  // 10^(-loss / 10) = 2^(sum x_s len_s)
+  const double att2 = -std::log2(10.0) / 10.0 / 1000.0;
+  for (int i = 0; i < std::min(a.ni, kLeanMax); ++i) {
+    OnePlane &O = k.pl[i];
+    const ss_interface &I = a.ifc[i];
     double mn[3];
     for (int j = 0; j < 3; ++j) {
       mn[j] = I.mean_normal[j];
@@ -57,25 +59,32 @@ RefSplitConsts split_consts(const RefArgs &a) {
       O.c4l[c] = cd.lo;
       O.cn[c] = (float)(I.coef[c] * mn[0] + I.coef[2 + c] * mn[1]);
     }
-    const double n1 = a.n_leg[0], n2 = a.n_leg[1];
+    const double n1 = a.n_leg[i], n2 = a.n_leg[i + 1];
     O.up = n1 <= n2;
     const double r = std::min(n1, n2) / std::max(n1, n2);
     O.r = (float)r;
     O.k2 = (float)(-0.5 * (1.0 - r * r));
     O.k4 = (float)(-0.125 * (1.0 - r * r) * (1.0 + 3.0 * r * r));
     O.vec = (reinterpret_cast<uintptr_t>(I.table) & 7) == 0;
+  }
+  {
     OneLegs &l = k.legs;
-    const df d1 = df_from_double(n1), d2 = df_from_double(n2);
+    const df d1 = df_from_double(a.n_leg[0]), d2 = df_from_double(a.n_leg[1]);
     l.n1 = d1.hi;
     l.n1l = d1.lo;
     l.n2 = d2.hi;
     l.n2l = d2.lo;
-    l.i1 = (float)(1.0 / n1);
-    l.i2 = (float)(1.0 / n2);
-    // 10^(-loss / 10) = 2^(x1 s1 + x2 s2)
-    const double x = -std::log2(10.0) / 10.0 / 1000.0;
-    l.x1 = (float)(x * a.att_leg[0]);
-    l.x2 = (float)(x * a.att_leg[1]);
+    l.i1 = (float)(1.0 / a.n_leg[0]);
+    l.i2 = (float)(1.0 / a.n_leg[1]);
+    l.x1 = (float)(att2 * a.att_leg[0]);
+    l.x2 = (float)(att2 * a.att_leg[1]);
+  }
+  for (int i = 0; i <= std::min(a.leg_last, kLeanMax); ++i) {
+    const df n = df_from_double(a.n_leg[i]);
+    k.lean.n[i] = n.hi;
+    k.lean.nl[i] = n.lo;
+    k.lean.inv[i] = (float)(1.0 / a.n_leg[i]);
+    k.lean.x[i] = (float)(att2 * a.att_leg[i]);
   }
   for (int i = 0; i <= a.leg_last; ++i) {
     const df n = df_from_double(a.n_leg[i]);
@@ -110,22 +119,37 @@ RefSplitConsts split_consts(const RefArgs &a) {
   return k;
 }
 
-bool one_crossing(const RefArgs &a) {
-  if (a.joint || a.ni != 1 || a.leg_last != 1) return false;
+// What the single-crossing and lean joint paths both ask for.
+static bool lean_common(const RefArgs &a) {
   if (a.F.gamma_f64 && a.F.sigma) return false;
-  for (int i = 0; i < 2; ++i)
+  for (int i = 0; i <= a.ni; ++i)
     if (!(std::fabs(a.n_leg[i] * a.n_leg[i] - a.eps_leg[i]) <=
           1e-9 * a.eps_leg[i]))
       return false;
   // cell indices are clamped as exact float32 integers
-  return a.ifc[0].ny < (1 << 22) && a.ifc[0].nx < (1 << 22);
+  for (int i = 0; i < a.ni; ++i)
+    if (a.ifc[i].ny >= (1 << 22) || a.ifc[i].nx >= (1 << 22)) return false;
+  return true;
+}
+
+bool one_crossing(const RefArgs &a) {
+  return !a.joint && a.ni == 1 && a.leg_last == 1 && lean_common(a);
+}
+
+bool lean_joint(const RefArgs &a) {
+  // (a histogram beyond the usual budget leaves no room for the constants)
+  return (size_t)a.n_seg * sizeof(float2) <= 96 * 1024 && a.joint && a.ni <= kLeanMax && a.n_newton >= 3 &&
+         a.n_backtrack >= 1 && !a.rough_cross && lean_common(a);
 }
 
 // Dynamic shared memory of the fast kernel: the trace block's histograms
 // and the series table.
 size_t split_smem_bytes(const RefArgs &a, int tb) {
   return (size_t)tb * a.n_seg * sizeof(float2) +
-         (a.rough_kind ? (a.n_terms + 1) * sizeof(float) : 0);
+         (a.rough_kind ? (a.n_terms + 1) * sizeof(float) : 0) +
+         (lean_joint(a) ? (size_t)a.ni * kOnePerIface * kSplitThreads *
+                              sizeof(float)
+                        : 0);
 }
 
 int refracted_split_launch(RefArgs &a, const Plan &p, cudaStream_t st) {

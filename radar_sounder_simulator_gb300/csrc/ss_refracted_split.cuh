@@ -48,7 +48,7 @@
 #include "ss_df.cuh"
 #include "ss_f32.cuh"
 #include "ss_refracted_fp64.cuh"
-#include "ss_refracted_one.cuh"
+#include "ss_refracted_lean.cuh"
 
 namespace ss {
 
@@ -64,9 +64,18 @@ constexpr float kLookupGuard = 1.5e-4f;
 constexpr float kBinGuard = 1e-6f;
 constexpr double kOplGuardChain = 5e-5;
 // Path-class argument of the kernels: 0 the sequential chain, 1-4 and
-// kDeepNI the joint solve through that many interfaces, kOneNI the
-// sequential solve of a single crossing (ss_refracted_one.cuh).
+// kDeepNI the joint solve through that many interfaces in its general form,
+// kOneNI the sequential solve of a single crossing (ss_refracted_one.cuh),
+// kOneNI - n the joint solve through n = 1..kLeanMax interfaces in its lean
+// form (ss_refracted_lean.cuh).
 constexpr int kOneNI = -1;
+constexpr int lean_class(int n) { return kOneNI - n; }
+// Interfaces of a lean class (0 for the others), and the general class that
+// evaluates its deferred pairs.
+constexpr int lean_count(int NI) { return NI < kOneNI ? kOneNI - NI : 0; }
+constexpr int general_class(int NI) {
+  return NI == kOneNI ? 0 : NI < kOneNI ? kOneNI - NI : NI;
+}
 
 // Per-interface constants of the float32 lookup pass.
 struct MeanPlane32 {
@@ -91,8 +100,9 @@ struct RefSplitConsts {
   // rate is the differentiated parameter
   float att_mask[SS_MAX_IFACE + 1];
   MeanPlane32 mean[SS_MAX_IFACE];
-  OnePlane one;   // single-crossing path (kOneNI)
-  OneLegs legs;
+  OnePlane pl[kLeanMax];  // single-crossing and lean joint paths
+  OneLegs legs;           // single crossing
+  LeanLegs lean;          // lean joint path
 };
 
 __device__ __forceinline__ float dot3a(const float *a, const float *b) {
@@ -1189,11 +1199,12 @@ __device__ __forceinline__ bool pair_eval(
     const double *p64, const float *u, const float *pv, const float *pat,
     int pa_len, const float *lg, const float *fad, int i, const float *q,
     PairOut &o, PairGrad *pg = nullptr) {
+  constexpr int GI = general_class(NI);
   PathS P;
-  if (NI <= 0)
+  if (GI == 0)
     path_sequential_split<EXACT, GRAD>(a, k, T, p64, q, P);
   else
-    path_joint_split<NI <= 0 ? 1 : NI, EXACT, GRAD>(a, k, T, p64, q, P);
+    path_joint_split<GI == 0 ? 1 : GI, EXACT, GRAD>(a, k, T, p64, q, P);
   if (!EXACT && P.defer) return false;
   PairGeo G;
   path_geo(a, k, P, GRAD, G);
@@ -1204,7 +1215,7 @@ __device__ __forceinline__ bool pair_eval(
         if (!EXACT) return false;
         bool v64;
         const double q64[3] = {q[0], q[1], q[2]};
-        const double o64 = full_opl64<NI <= 0 ? 0 : NI>(a, p64, q64, v64);
+        const double o64 = full_opl64<GI>(a, p64, q64, v64);
         const double twtt = __ddiv_rn(__dmul_rn(2.0, o64), a.c);
         fb = (float)floor(__ddiv_rn(__dsub_rn(twtt, a.t0), a.dt));
         return true;
@@ -1224,10 +1235,11 @@ __device__ __forceinline__ bool pair_one(
   const float4 A = tr[0];
   one_offset(A, make_float2(tr[1].x, tr[1].y), f.q, Ph, Pl);
   int cell;
-  if (!one_cell(k.one, m, Ph, a.ifc[0].ny, a.ifc[0].nx, cell))
+  float v0[3];
+  if (!one_cell(k.pl[0], m, Ph, a.ifc[0].ny, a.ifc[0].nx, 1.0f, cell, v0))
     return false;
   PairGeo G;
-  one_path(k.one, k.legs, a.ifc[0].table, cell, f.q, Ph, Pl, kTol32,
+  one_path(k.pl[0], k.legs, a.ifc[0].table, cell, f.q, Ph, Pl, kTol32,
                  G);
   if (a.rough_cross) {
     // c0 and c_last of the crossing again (a rarely used option)
@@ -1247,6 +1259,27 @@ __device__ __forceinline__ bool pair_one(
       [](float &) { return false; });
 }
 
+// The lean joint pair of a facet whose lookup constants are staged in `col`.
+template <int NI, int ROUGH, bool PLAIN>
+__device__ __forceinline__ bool pair_lean(
+    const RefArgs &a, const RefSplitConsts &k, const float4 *tr,
+    const float *u, const float *pv, const float *pat, int pa_len,
+    const float *lg, const float *fad, int i, const float *q,
+    const float *col, int stride, PairOut &o) {
+  constexpr int N = lean_count(NI) > 0 ? lean_count(NI) : 1;
+  const float4 A = tr[0];
+  const float2 B = make_float2(tr[1].x, tr[1].y);
+  PairGeo G;
+  if (!lean_path<N>(k.pl, k.lean, a.ifc, a.k_pad, a.n_newton, col, stride, q,
+                    A, B, kTol32, G))
+    return false;
+  const FacetAt f{a, k, i};
+  const float v[3] = {q[0] - A.x, q[1] - A.y, q[2] - A.z};
+  return pair_finish<ROUGH, false, PLAIN, true>(
+      a, k, f, G, v, u, pv, pat, pa_len, lg, fad, i, o, nullptr,
+      [](float &) { return false; });
+}
+
 // One CTA's work item of the fast kernel: facet chunk `chunk` of trace
 // block `group`; thread <-> facet; per-trace histograms in shared memory;
 // pairs that need a float64 decision are marked in the deferral bitmask
@@ -1259,6 +1292,9 @@ __device__ __forceinline__ void refracted_split_cta(const RefArgs &a,
                                                     unsigned char *smem_raw) {
   float2 *hist = reinterpret_cast<float2 *>(smem_raw);
   float *lg = reinterpret_cast<float *>(hist + (size_t)a.tb * a.n_seg);
+  // the lean joint path's facet constants, a column per thread
+  constexpr int LN = lean_count(NI);
+  float *col = lg + (ROUGH != SS_ROUGH_NONE ? a.n_terms + 1 : 0) + threadIdx.x;
   __shared__ double s_p64[SS_MAX_TB][3];
   __shared__ TraceS s_tr[SS_MAX_TB];
   __shared__ float4 s_t4[SS_MAX_TB][2];  // position hi, lo (kOneNI)
@@ -1277,7 +1313,7 @@ __device__ __forceinline__ void refracted_split_cta(const RefArgs &a,
   if (tid < nt) {
     const int t = t_base + tid;
     load_trace(a, t, s_tr[tid], s_p64[tid], s_u[tid], s_pv[tid]);
-    if (NI == kOneNI) stage_trace4(s_tr[tid], s_t4[tid]);
+    if (NI < 0) stage_trace4(s_tr[tid], s_t4[tid]);
     long lo = (long)a.off[t] * a.bs;
     long hi = min((long)(a.off[t] + a.n_win) * a.bs, (long)a.N);
     s_lo[tid] = (int)min(lo, (long)a.N);
@@ -1323,7 +1359,9 @@ __device__ __forceinline__ void refracted_split_cta(const RefArgs &a,
     f.q[0] = a.F.cx[i]; f.q[1] = a.F.cy[i]; f.q[2] = a.F.cz[i];
     if (NI == kOneNI) {
       load_facet<ROUGH>(a, k, i, f);
-      one_facet(k.one, f.q, m);
+      one_facet(k.pl[0], f.q, m);
+    } else if (LN > 0) {
+      lean_facet<LN>(k.pl, f.q, col, blockDim.x);
     }
     for (int tt = 0; tt < nt; ++tt) {
       if (i < s_lo[tt] || i >= s_hi[tt]) continue;
@@ -1333,6 +1371,10 @@ __device__ __forceinline__ void refracted_split_cta(const RefArgs &a,
         ok = pair_one<ROUGH, PLAIN>(a, k, s_t4[tt], s_u[tt], s_pv[tt],
                                            s_pat, pa_len, lg, s_fad, i, f, m,
                                            o);
+      else if (LN > 0)
+        ok = pair_lean<NI, ROUGH, PLAIN>(a, k, s_t4[tt], s_u[tt], s_pv[tt],
+                                         s_pat, pa_len, lg, s_fad, i, f.q,
+                                         col, blockDim.x, o);
       else
         ok = pair_eval<NI, ROUGH, false, false, PLAIN>(
             a, k, s_tr[tt], s_p64[tt], s_u[tt], s_pv[tt], s_pat, pa_len, lg,
@@ -1364,12 +1406,16 @@ __device__ __forceinline__ void refracted_split_cta(const RefArgs &a,
 }
 
 // Fast kernel: one CTA per (facet chunk, trace block).
-// Up to two crossings the solve fits 64 registers, so two 512-thread CTAs
-// share an SM (32 warps; the joint solve through two interfaces spills a
-// few words at that budget and still gains 8%); through three or more it
-// keeps ~125 registers and one CTA.
+// Up to two crossings the general solve fits 64 registers, so two 512-thread
+// CTAs share an SM (32 warps; the joint solve through two interfaces spills
+// a few words at that budget and still gains 8%); through three or more it
+// keeps ~125 registers and one CTA. The lean joint solve keeps one CTA from
+// two interfaces on (its lookup constants also take 20 KB and more).
+constexpr int split_ctas(int NI) {
+  return NI >= 3 || lean_count(NI) >= 2 ? 1 : 2;
+}
 template <int NI, int ROUGH, bool PLAIN>
-__global__ void __launch_bounds__(kSplitThreads, NI >= 3 ? 1 : 2)
+__global__ void __launch_bounds__(kSplitThreads, split_ctas(NI))
 refracted_split_kernel(RefArgs a, RefSplitConsts k) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   refracted_split_cta<NI, ROUGH, PLAIN>(a, k, blockIdx.x, blockIdx.y,
@@ -1506,8 +1552,8 @@ inline int launch_split(RefArgs &a, const RefSplitConsts &k, const Plan &p,
   const int blocks =
       (int)std::max<unsigned long long>(1, std::min<unsigned long long>(
                                                want, 8ull * sm_count()));
-  refracted_split_fixup<NI, ROUGH><<<blocks, 32 * kFixWarps, fsmem, st>>>(a,
-                                                                          k);
+  refracted_split_fixup<general_class(NI), ROUGH>
+      <<<blocks, 32 * kFixWarps, fsmem, st>>>(a, k);
   return cuda_status(cudaGetLastError(), "refracted_split fix-up launch");
 }
 
@@ -1556,7 +1602,7 @@ __device__ __forceinline__ int ref_batch_find(const RefBatchJob *jobs,
 }
 
 template <int NI, int ROUGH, bool PLAIN>
-__global__ void __launch_bounds__(kSplitThreads, NI >= 3 ? 1 : 2)
+__global__ void __launch_bounds__(kSplitThreads, split_ctas(NI))
 refracted_batch_kernel(const RefBatchJob *jobs, int n_jobs,
                        long long n_items, unsigned long long *counter) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1658,6 +1704,10 @@ refracted_batch_fixup(const RefBatchJob *jobs, int n_jobs,
                                       size_t smem);
 SS_REF_BATCH_DECL(0)
 SS_REF_BATCH_DECL(one)
+SS_REF_BATCH_DECL(lean1)
+SS_REF_BATCH_DECL(lean2)
+SS_REF_BATCH_DECL(lean3)
+SS_REF_BATCH_DECL(lean4)
 SS_REF_BATCH_DECL(1)
 SS_REF_BATCH_DECL(2)
 SS_REF_BATCH_DECL(3)
@@ -1679,8 +1729,8 @@ inline int ref_batch_launch_t(const RefBatchJob *jobs, int n_jobs,
       ((unsigned long long)n_words + 32 * kFixWarps - 1) / (32 * kFixWarps);
   const int blocks = (int)std::max<unsigned long long>(
       1, std::min<unsigned long long>(want, 8ull * sm_count()));
-  refracted_batch_fixup<NI, ROUGH><<<blocks, 32 * kFixWarps, fix_smem, st>>>(
-      jobs, n_jobs, n_words);
+  refracted_batch_fixup<general_class(NI), ROUGH>
+      <<<blocks, 32 * kFixWarps, fix_smem, st>>>(jobs, n_jobs, n_words);
   return cuda_status(cudaGetLastError(), "refracted batch fix-up launch");
 }
 
@@ -1752,6 +1802,10 @@ size_t split_smem_bytes(const RefArgs &a, int tb);
 // gradient sums its traces with a hundredfold cancellation, which shows any
 // change of the pairs' float32 rounding at 1e-3 of a weak gradient.
 bool one_crossing(const RefArgs &a);
+
+// Whether the call takes the lean joint path: up to kLeanMax interfaces, a
+// Newton budget that lets it converge, and the same conditions.
+bool lean_joint(const RefArgs &a);
 
 // Fast + fix-up launches of one crossed-interface count (NI = 0: the
 // sequential path; one: a single crossing), each instantiated in its own

@@ -5,7 +5,8 @@ namespace ss {
 
 int split_launch_ni2(RefArgs &a, const RefSplitConsts &k, const Plan &p,
                      size_t smem, cudaStream_t st) {
-  return launch_split_r<2>(a, k, p, smem, st);
+  return lean_joint(a) ? launch_split_r<lean_class(2)>(a, k, p, smem, st)
+                       : launch_split_r<2>(a, k, p, smem, st);
 }
 
 int refracted_batch_launch_ni2(const RefBatchJob *jobs, int n_jobs,
@@ -19,6 +20,22 @@ int refracted_batch_launch_ni2(const RefBatchJob *jobs, int n_jobs,
 
 int refracted_batch_occupancy_ni2(int rough_kind, bool plain, size_t smem) {
   return ref_batch_occupancy<2>(rough_kind, plain, smem);
+}
+
+int refracted_batch_launch_nilean2(const RefBatchJob *jobs, int n_jobs,
+                                   long long n_items, long long n_words,
+                                   unsigned long long *counter,
+                                   int rough_kind, bool plain, int ctas,
+                                   size_t smem, size_t fix_smem,
+                                   cudaStream_t st) {
+  return ref_batch_launch_r<lean_class(2)>(jobs, n_jobs, n_items, n_words,
+                                           counter, rough_kind, plain, ctas,
+                                           smem, fix_smem, st);
+}
+
+int refracted_batch_occupancy_nilean2(int rough_kind, bool plain,
+                                      size_t smem) {
+  return ref_batch_occupancy<lean_class(2)>(rough_kind, plain, smem);
 }
 
 }  // namespace ss
