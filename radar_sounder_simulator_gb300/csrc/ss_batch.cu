@@ -26,6 +26,7 @@ namespace ss {
 static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 struct BatchLayout {
+  int form = kFormPlain;  // the widest form any job needs
   std::vector<BatchJob> jobs;
   size_t table_off = 256, bytes = 0, smem = 0;
   long long n_items = 0, n_out = 0;
@@ -72,6 +73,7 @@ static int batch_layout(const ss_coherent_job *jobs, int n_jobs,
                 "kind");
       return SS_ERR_ARG;
     }
+    L.form = std::min(L.form, coherent_form(a));
     if (threads == 512 &&
         (a.precision == SS_PREC_FP64 || a.rough_kind != SS_ROUGH_NONE)) {
       set_error("512-thread batches take smooth split-precision jobs only");
@@ -190,8 +192,8 @@ extern "C" int ss_coherent_batch_prepare(const ss_coherent_job *jobs,
   }
   int per_sm = L.precision == SS_PREC_FP64
                    ? batch_fp64_blocks_per_sm(L.threads, L.smem)
-                   : batch_split_blocks_per_sm(L.rough_kind, L.threads,
-                                               L.smem);
+                   : batch_split_blocks_per_sm(L.rough_kind, L.form,
+                                               L.threads, L.smem);
   if (per_sm <= 0) {
     set_error("batched kernel does not fit on an SM with this shared memory");
     return SS_ERR_UNSUPPORTED;
@@ -206,6 +208,7 @@ extern "C" int ss_coherent_batch_prepare(const ss_coherent_job *jobs,
   info->precision = L.precision;
   info->rough_kind = L.rough_kind;
   info->threads = L.threads;
+  info->reserved = L.form;  // the kernel form every job fits
   info->ctas = per_sm * sm_count();
   info->n_items = L.n_items;
   info->n_out = L.n_out;
@@ -234,8 +237,9 @@ extern "C" int ss_coherent_batch_run(const ss_batch_info *info,
                                            info->smem, st)
               : coherent_batch_split_launch(jobs, info->n_jobs,
                                             info->n_items, counter,
-                                            info->rough_kind, info->threads,
-                                            info->ctas, info->smem, st);
+                                            info->rough_kind, info->reserved,
+                                            info->threads, info->ctas,
+                                            info->smem, st);
   if (s) return s;
   return batch_reduce_launch(jobs, info->n_jobs, info->n_out, f64, st);
 }

@@ -22,6 +22,11 @@ struct CoArgs {
   double *part_drop;   // (n_chunks, T) partial dropped power
 };
 
+// Instantiation of the split kernels a smooth call takes: every option, none
+// but an antenna pattern, none at all (see ss_coherent_split.cu).
+enum { kFormAny = 0, kFormBeam = 1, kFormPlain = 2 };
+int coherent_form(const CoArgs &a);
+
 int coherent_plan(const ss_coherent_opts *o, int T, int N, Plan *p,
                   bool rough);
 size_t coherent_scratch(const ss_coherent_opts *o, int T, int N);
@@ -31,16 +36,16 @@ int build_co_args(const ss_coherent_opts *opts, const ss_facets *facets,
                   const ss_roughness *rough, const ss_output *out, Plan &p,
                   CoArgs &a);
 
-// Shared-memory histograms of the split coherent kernel: planar real and
-// imaginary planes of `tb` traces each, a trace's row padded to n_seg + 11
-// floats so the block's traces start 11 banks apart (neighbouring facets
-// of a warp, spread over the traces, then rarely meet in one bank).
+// Shared-memory histograms of the split coherent kernel: (re, im) bins of
+// `tb` traces, a trace's row padded to n_seg + 5 bins so the block's traces
+// start ten banks apart (neighbouring facets of a warp, spread over the
+// traces, then rarely meet in one bank).
 __host__ __device__ __forceinline__ int split_hist_stride(int n_seg) {
-  return n_seg + 11;
+  return n_seg + 5;
 }
 __host__ __device__ __forceinline__ size_t split_hist_bytes(int n_seg,
                                                             int tb) {
-  return (size_t)2 * tb * split_hist_stride(n_seg) * sizeof(float);
+  return (size_t)tb * split_hist_stride(n_seg) * sizeof(float2);
 }
 
 // float32 / double-float constants of the split coherent kernel.
@@ -69,13 +74,14 @@ struct BatchJob {
 int coherent_batch_split_launch(const BatchJob *jobs, int n_jobs,
                                 long long n_items,
                                 unsigned long long *counter, int rough_kind,
-                                int threads, int ctas, size_t smem,
+                                int form, int threads, int ctas, size_t smem,
                                 cudaStream_t st);
 int coherent_batch_fp64_launch(const BatchJob *jobs, int n_jobs,
                                long long n_items, unsigned long long *counter,
                                int threads, int ctas, size_t smem,
                                cudaStream_t st);
-int batch_split_blocks_per_sm(int rough_kind, int threads, size_t smem);
+int batch_split_blocks_per_sm(int rough_kind, int form, int threads,
+                              size_t smem);
 int batch_fp64_blocks_per_sm(int threads, size_t smem);
 // Ordered chunk reduction of every job's partials into its output.
 int batch_reduce_launch(const BatchJob *jobs, int n_jobs, long long n_out,

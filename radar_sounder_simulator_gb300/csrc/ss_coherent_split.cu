@@ -13,18 +13,18 @@
 //     exact), its bin position split into an integer and a fraction, and the
 //     products of q = p_c - c with the facet's normal and edge vectors.
 //   * Per trace t of the block, with w = p_t - p_c (a few trace spacings):
-//     r_t^2 - r_c^2 = 2 q.w + |w|^2 = N, so r_t - r_c = N / (r_c + r_t).
-//     Within a block the track is straight to well under a metre, so
-//     w = lam u + eps with u the block's track direction: q.u is formed
-//     once per facet as a double-float, and N = 2 (lam q.u + q.eps) +
-//     |w|^2 takes one exact product per pair (q.eps, |eps| < 1 m, in
-//     float32). N is thus a double-float; the division
-//     takes a float32 quotient and one correction against the double-float
-//     denominator 2 r_c + dr, so dr = r_t - r_c is good to ~2e-11 of its
-//     size (3e-9 m at |w| = 160 m; a float32 dr would carry ulp(|w|)/2 of
-//     rounding: 4e-6 m at 100 m, 8e-5 rad of phase at 450 MHz). The middle
-//     trace has w = 0 and its pairs are exact to the reference's
-//     double-float.
+//     r_t^2 - r_c^2 = 2 q.w + |w|^2 = N, so dr = r_t - r_c solves
+//     dr^2 + 2 r_c dr = N. Within a block the track is straight to well
+//     under a metre, so w = lam u + eps with u the block's track direction:
+//     q.u is formed once per facet as a double-float, and N = 2 (lam q.u +
+//     q.eps) + |w|^2 takes one exact product per pair (q.eps, |eps| < 1 m,
+//     in float32). N is thus a double-float; dr is the float32 difference
+//     of the two ranges (right to an ulp of the range) and one Newton step
+//     of that equation, whose residual is formed exactly and whose slope is
+//     2 r_t: no division, and dr good to ~2e-11 of its size (3e-9 m at
+//     |w| = 160 m; a float32 dr would carry ulp(|w|)/2 of rounding: 4e-6 m
+//     at 100 m, 8e-5 rad of phase at 450 MHz). The middle trace has w = 0
+//     and its pairs are exact to the reference's double-float.
 //
 // The bin position ubc + fc + A dr is then good to ~2e-7 bins; a pair
 // within 2e-6 bins of an edge recomputes its own double-float range and
@@ -38,7 +38,16 @@
 // Everything else (incidence, sincs, taper, antenna gain, roughness series)
 // runs in float32 from q + w and the facet's per-block products;
 // histograms accumulate float32 per CTA chunk and the reduce kernel sums
-// the chunks by float32 two-sums (~2^-48 relative).
+// the chunks by float32 two-sums (~2^-48 relative). A bin is one 8-byte
+// (re, im) cell updated by a 64-bit compare-and-swap (hist_add): one shared
+// round trip per pair where two float atomics -- loops of 32-bit
+// compare-and-swaps in shared memory -- took two.
+//
+// Bound by instruction issue, ~240 instructions per pair (307 with a
+// division for dr, two atomics and denormal handling in the special
+// functions): 512^2 facets x 1024 traces with an antenna pattern 2.45 ->
+// 1.85 ms; 128^2 x 256, which is half set-up and reduce, 133 -> 104 us with
+// both.
 #include <algorithm>
 
 #include "ss_coherent.cuh"
@@ -66,15 +75,19 @@ __device__ __forceinline__ int small_int(float x) {
 // One CTA's work item: facet chunk `chunk` of trace block `group`. Shared
 // by the one-call kernel (item = block index) and the batched persistent
 // kernel (item pulled from a work queue).
-template <int ROUGH>
+// FORM: kFormPlain -- isotropic antenna, no taper, no side split, whole bins;
+// kFormBeam -- the same with an antenna pattern; kFormAny -- every option.
+// The options cost registers and uniform branches whether used or not (512^2
+// facets x 1024 traces, sum alone: 2.45 ms with them, 1.90 ms without).
+template <int ROUGH, bool BATCH, int FORM>
 __device__ __forceinline__ void coherent_split_cta(const CoArgs &a,
                                                    const SplitConsts &k,
                                                    int chunk, int group,
                                                    unsigned char *smem_raw) {
   const int hs = split_hist_stride(a.n_seg);
-  float *hre = reinterpret_cast<float *>(smem_raw);
-  float *him = hre + (size_t)a.tb * hs;
-  float *inv = him + (size_t)a.tb * hs;  // 1/m of the series (rough only)
+  float2 *hist = reinterpret_cast<float2 *>(smem_raw);
+  float *inv =  // 1/m of the series (rough only)
+      reinterpret_cast<float *>(hist + (size_t)a.tb * hs);
   __shared__ float s_ph[SS_MAX_TB][3], s_pl[SS_MAX_TB][3];
   __shared__ double s_p64[SS_MAX_TB][3];
   // trace offsets w = p_t - p_c = lam u + eps, u the block's track
@@ -131,58 +144,65 @@ __device__ __forceinline__ void coherent_split_cta(const CoArgs &a,
     s_pat[pa_len + j] = (float)a.pb[j];
   if (ROUGH == SS_ROUGH_GAUSS_FULL && tid < SS_FAD_N)
     s_fad[tid] = (float)a.fad.a[tid];
-  for (int j = tid; j < 2 * a.tb * hs; j += blockDim.x) hre[j] = 0.0f;
   if (ROUGH != SS_ROUGH_NONE) fill_inv_table(inv, a.n_terms, tid, blockDim.x);
   __syncthreads();
   if (a.pat_kind == SS_PAT_TABULATED)
     tab_slopes(a.pat_n, s_pat, s_pat + pa_len, s_slope, &s_tinv, tid,
                blockDim.x);
-  if (tid == 0) {
-    int lo = s_win[0].x, hi = s_win[0].y;
-    for (int j = 1; j < nt; ++j) {
-      lo = min(lo, s_win[j].x);
-      hi = max(hi, s_win[j].y);
-    }
-    long len = max(hi - lo, 0);
-    s_rng[0] = lo + (int)(len * chunk / a.n_chunks);
-    s_rng[1] = lo + (int)(len * (chunk + 1) / a.n_chunks);
-    s_next = s_rng[0];
-    // track direction u of the block (first to last trace) and each
-    // trace's offset w = lam u + eps from the middle trace, in float64
-    const int c = nt / 2;
-    double u[3], un = 0.0;
+  // The first warp sets the block up while the others clear the histograms
+  // (its float64 operations come out one at a time: done by one thread for
+  // all traces they held a 128^2 facet x 256 trace call's CTAs for 4 us).
+  // Thread t: the track direction u of the block (first to last trace) and
+  // its trace's offset w = lam u + eps from the middle trace, in float64.
+  if (tid < 32) {
+    const int c = nt / 2, t = min(tid, nt - 1);
+    double u[3], w[3], un = 0.0, w2 = 0.0, lam = 0.0, e2 = 0.0;
     for (int j = 0; j < 3; ++j) {
       u[j] = s_p64[nt - 1][j] - s_p64[0][j];
       un += u[j] * u[j];
+      w[j] = s_p64[t][j] - s_p64[c][j];
+      w2 += w[j] * w[j];
     }
     un = sqrt(un);
-    for (int j = 0; j < 3; ++j) u[j] = un > 0.0 ? u[j] / un : (j == 0);
-    double wmax = 0.0, emax = 0.0;
-    for (int t = 0; t < nt; ++t) {
-      double w[3], lam = 0.0, e2 = 0.0;
-      for (int j = 0; j < 3; ++j) {
-        w[j] = s_p64[t][j] - s_p64[c][j];
-        lam += w[j] * u[j];
-      }
-      float e[3];
-      for (int j = 0; j < 3; ++j) {
-        const double ej = w[j] - lam * u[j];
-        e[j] = (float)ej;
-        e2 += ej * ej;
-      }
+    const double iu = un > 0.0 ? 1.0 / un : 0.0;
+    for (int j = 0; j < 3; ++j) {
+      u[j] = un > 0.0 ? u[j] * iu : (j == 0);
+      lam += w[j] * u[j];
+    }
+    float e[3];
+    for (int j = 0; j < 3; ++j) {
+      const double ej = w[j] - lam * u[j];
+      e[j] = (float)ej;
+      e2 += ej * ej;
+    }
+    const bool wide = w2 > (double)kWideBlock * kWideBlock ||
+                      e2 > kBlockBend * kBlockBend;
+    const bool any = __any_sync(0xffffffffu, wide);
+    if (tid < nt) {
       const float lh = (float)lam;
       s_lw[t].x = lh;
       s_lw[t].y = (float)(lam - (double)lh);
       s_we[t] = make_float4(e[0], e[1], e[2], 0.0f);
-      wmax = fmax(wmax, sqrt(w[0] * w[0] + w[1] * w[1] + w[2] * w[2]));
-      emax = fmax(emax, sqrt(e2));
     }
-    for (int j = 0; j < 3; ++j) {
-      s_tu[j] = (float)u[j];
-      s_tu[3 + j] = (float)(u[j] - (double)s_tu[j]);
+    if (tid == 0) {
+      for (int j = 0; j < 3; ++j) {
+        s_tu[j] = (float)u[j];
+        s_tu[3 + j] = (float)(u[j] - (double)s_tu[j]);
+      }
+      s_ref = any ? -1 : c;
+      int lo = s_win[0].x, hi = s_win[0].y;
+      for (int j = 1; j < nt; ++j) {
+        lo = min(lo, s_win[j].x);
+        hi = max(hi, s_win[j].y);
+      }
+      long len = max(hi - lo, 0);
+      s_rng[0] = lo + (int)(len * chunk / a.n_chunks);
+      s_rng[1] = lo + (int)(len * (chunk + 1) / a.n_chunks);
+      s_next = s_rng[0];
     }
-    s_ref = wmax <= kWideBlock && emax <= kBlockBend ? c : -1;
   }
+  for (int j = tid; j < a.tb * hs; j += blockDim.x)
+    hist[j] = make_float2(0.0f, 0.0f);
   __syncthreads();
 
   const float nsf = (float)a.n_samples;
@@ -207,7 +227,7 @@ __device__ __forceinline__ void coherent_split_cta(const CoArgs &a,
     if (base >= i_end) break;
     const int i = base + lane;
     if (i >= i_end) continue;
-    const float cx = a.F.cx[i], cy = a.F.cy[i], cz = a.F.cz[i];
+    const float cx0 = a.F.cx[i], cy0 = a.F.cy[i], cz0 = a.F.cz[i];
     const float nx = a.F.nx[i], ny = a.F.ny[i], nz = a.F.nz[i];
     const float e1x = a.F.e1x[i], e1y = a.F.e1y[i], e1z = a.F.e1z[i];
     const float e2x = a.F.e2x[i], e2y = a.F.e2y[i], e2z = a.F.e2z[i];
@@ -230,11 +250,11 @@ __device__ __forceinline__ void coherent_split_cta(const CoArgs &a,
     float quh, qul;                               // q.u as a double-float
     auto reference = [&](int j) {
       float e;
-      two_sum(s_ph[j][0], -cx, qhx, e);
+      two_sum(s_ph[j][0], -cx0, qhx, e);
       fast_two_sum(qhx, e + s_pl[j][0], qhx, qlx);
-      two_sum(s_ph[j][1], -cy, qhy, e);
+      two_sum(s_ph[j][1], -cy0, qhy, e);
       fast_two_sum(qhy, e + s_pl[j][1], qhy, qly);
-      two_sum(s_ph[j][2], -cz, qhz, e);
+      two_sum(s_ph[j][2], -cz0, qhz, e);
       fast_two_sum(qhz, e + s_pl[j][2], qhz, qlz);
       // S = |q|^2 (double-float), r_c = sqrt(S): rsqrt + one Newton step
       float sx, ex, sy, ey, sz, ez, s1, e1_, Sh, e2_;
@@ -279,7 +299,7 @@ __device__ __forceinline__ void coherent_split_cta(const CoArgs &a,
       const float c0 = qnh * yc;
       const float ce = __fmaf_rn(-c0, rch, qnh) + qnl - c0 * rcl;
       cosc = __fmaf_rn(ce, yc, c0);
-      if (a.taper) {
+      if (FORM == kFormAny && a.taper) {
         xnx = __fmaf_rn(qhy, nz, -qhz * ny) + __fmaf_rn(qly, nz, -qlz * ny);
         xny = __fmaf_rn(qhz, nx, -qhx * nz) + __fmaf_rn(qlz, nx, -qlx * nz);
         xnz = __fmaf_rn(qhx, ny, -qhy * nx) + __fmaf_rn(qlx, ny, -qly * nx);
@@ -313,6 +333,12 @@ __device__ __forceinline__ void coherent_split_cta(const CoArgs &a,
     // bins from the exact u) runs only within 1e-8 bins of an edge, where
     // the two could round differently.
     auto exact_bin = [&](int tt, float &fb, float &frac) {
+      // (the one-call kernel reads the centroid again: held through the loop
+      // it spilled; the batch kernel, which addresses its job's arrays
+      // through memory, spills less with it held)
+      const float cx = BATCH ? cx0 : a.F.cx[i];
+      const float cy = BATCH ? cy0 : a.F.cy[i];
+      const float cz = BATCH ? cz0 : a.F.cz[i];
       float dxh, dxl, dyh, dyl, dzh, dzl, e;
       two_sum(s_ph[tt][0], -cx, dxh, e);
       fast_two_sum(dxh, e + s_pl[tt][0], dxh, dxl);
@@ -373,30 +399,28 @@ __device__ __forceinline__ void coherent_split_cta(const CoArgs &a,
       float Nh, g;
       two_sum(2.0f * pq, __fmaf_rn(2.0f, lo, w.w), Nh, g);
       const float Nl = g + lw.z;
-      // float32 r_t for the amplitude and a first dr, then dr = N / D with
-      // D = r_c + r_t = 2 r_c + dr as a double-float and one correction:
-      // dr is then good to ~2e-11 of its size
+      // float32 r_t; dr = r_t - r_c to its rounding, then one Newton step of
+      // dr^2 + 2 r_c dr = N from the exact residual: the step carries the
+      // low part (up to an ulp of r), and dr is good to ~1e-10 m
       const float rr = __fmaf_rn(rch, rch, Nh);
-      const float inv_r = rsqrtf(rr);
-      const float dr0 = __fdividef(Nh, rch + rr * inv_r);
+      const float inv_r = rsq_n(rr);
+      const float dr = __fmaf_rn(rr, inv_r, -rch);
       float Dh, De;
-      fast_two_sum(2.0f * rch, dr0, Dh, De);
+      fast_two_sum(2.0f * rch, dr, Dh, De);
       const float Dl = __fmaf_rn(2.0f, rcl, De);
-      const float iD = __fdividef(1.0f, Dh);
-      const float dr = Nh * iD;
-      const float drl =
-          (__fmaf_rn(-dr, Dh, Nh) + __fmaf_rn(-dr, Dl, Nl)) * iD;
+      const float drl = (__fmaf_rn(-dr, Dh, Nh) + __fmaf_rn(-dr, Dl, Nl)) *
+                        (0.5f * inv_r);
       // --- amplitude (float32) ---
       // cos_t = (q.n + w.n) / r_t = cos_c + (w.n - cos_c dr) / r_t
       const float cosv = __fmaf_rn(
-          __fmaf_rn(-cosc, dr, dot3f(nx, ny, nz, w.x, w.y, w.z)), inv_r,
+          __fmaf_rn(-cosc, dr + drl, dot3f(nx, ny, nz, w.x, w.y, w.z)), inv_r,
           cosc);
       const float d1 = (qe1 + dot3f(e1x, e1y, e1z, w.x, w.y, w.z)) * inv_r;
       const float d2 = (qe2 + dot3f(e2x, e2y, e2z, w.x, w.y, w.z)) * inv_r;
       const float inv_r2 = inv_r * inv_r;
-      float amp = amp_f * cosv * sinc32(k.k * d1) * sinc32(k.k * d2) *
+      float amp = amp_f * cosv * sinc_n(k.k * d1) * sinc_n(k.k * d2) *
                   inv_r2;
-      if (a.taper) {
+      if (FORM == kFormAny && a.taper) {
         // tan^2 = sin^2 / cos^2 with sin^2 = |(q + w) x n|^2 / r_t^2 (no
         // 1 - cos^2 cancellation near nadir)
         const float sx = xnx + __fmaf_rn(w.y, nz, -w.z * ny);
@@ -427,12 +451,11 @@ __device__ __forceinline__ void coherent_split_cta(const CoArgs &a,
       const float n2 = rintf(pp * 0.159154943091895336f);
       float red = __fmaf_rn(-n2, 6.28318548202514648f, pp);
       red = __fmaf_rn(-n2, -1.74845553146951e-07f, red) + (pe + phc);
-      float sn, cs;
-      __sincosf(red, &sn, &cs);
+      const float sn = sin_n(red), cs = cos_n(red);
       float re = cr * sn - ci * cs;
       float im = cr * cs + ci * sn;
       const float qtx = qhx + w.x, qty = qhy + w.y, qtz = qhz + w.z;
-      if (a.pat_kind != SS_PAT_ISOTROPIC) {
+      if (FORM != kFormPlain && a.pat_kind != SS_PAT_ISOTROPIC) {
         const float g =
             a.pat_kind == SS_PAT_TABULATED
                 ? gain_tab32(a.pat_n, s_pat, s_pat + pa_len, s_slope, s_tinv,
@@ -456,29 +479,25 @@ __device__ __forceinline__ void coherent_split_cta(const CoArgs &a,
           fb < nsf + 4.0f)
         exact_bin(tt, fb, frac);
       int side_off = 0;
-      if (a.split &&
+      if (FORM == kFormAny && a.split &&
           dot3f(-qtx, -qty, -qtz, s_u[tt][0], s_u[tt][1], s_u[tt][2]) > 0.0f)
         side_off = a.n_samples;
       const int row = tt * hs + side_off;
       float drop = 0.0f;
-      if (a.interp) {
+      if (FORM == kFormAny && a.interp) {
         const float wq[2] = {1.0f - frac, frac};
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
           const float bq = fb + (float)q;
           const float pr = re * wq[q], pim = im * wq[q];
           if (bq >= 0.0f && bq < nsf) {
-            const int j = row + small_int(bq);
-            atomicAdd(hre + j, pr);
-            atomicAdd(him + j, pim);
+            hist_add(hist + row + small_int(bq), pr, pim);
           } else {
             drop += pr * pr + pim * pim;
           }
         }
       } else if (fb >= 0.0f && fb < nsf) {
-        const int j = row + small_int(fb);
-        atomicAdd(hre + j, re);
-        atomicAdd(him + j, im);
+        hist_add(hist + row + small_int(fb), re, im);
       } else {
         drop = re * re + im * im;
       }
@@ -519,7 +538,7 @@ __device__ __forceinline__ void coherent_split_cta(const CoArgs &a,
   for (int tt = 0; tt < nt; ++tt) {
     const size_t base = ((size_t)chunk * a.T + t_base + tt) * a.n_seg;
     for (int j = tid; j < a.n_seg; j += blockDim.x)
-      part[base + j] = make_float2(hre[tt * hs + j], him[tt * hs + j]);
+      part[base + j] = hist[tt * hs + j];
   }
   if (tid < nt)
     a.part_drop[(size_t)chunk * a.T + t_base + tid] = (double)s_drop[tid];
@@ -531,11 +550,12 @@ __device__ __forceinline__ void coherent_split_cta(const CoArgs &a,
 #define SS_SPLIT_MAXT(R) ((R) == SS_ROUGH_NONE ? 512 : 256)
 #define SS_SPLIT_MINB(R) ((R) == SS_ROUGH_NONE ? 2 : 3)
 
-template <int ROUGH>
+template <int ROUGH, int FORM>
 __global__ void __launch_bounds__(SS_SPLIT_MAXT(ROUGH), SS_SPLIT_MINB(ROUGH))
 coherent_split_kernel(CoArgs a, SplitConsts k) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  coherent_split_cta<ROUGH>(a, k, blockIdx.x, blockIdx.y, smem_raw);
+  coherent_split_cta<ROUGH, false, FORM>(a, k, blockIdx.x, blockIdx.y,
+                                         smem_raw);
 }
 
 // Batched persistent kernel: CTAs pull (job, trace block, facet chunk)
@@ -544,7 +564,7 @@ coherent_split_kernel(CoArgs a, SplitConsts k) {
 // MAXT = 512 (smooth facets only, 64 registers, two CTAs per SM) and
 // MAXT = 256 (80 registers, three CTAs per SM, no spills); the batch's CTA
 // size picks one, and the autotuner times both.
-template <int ROUGH, int MAXT>
+template <int ROUGH, int MAXT, int FORM>
 __global__ void __launch_bounds__(MAXT, MAXT == 512 ? 2 : 3)
 coherent_batch_split_kernel(const BatchJob *jobs, int n_jobs,
                             long long n_items, unsigned long long *counter) {
@@ -563,42 +583,56 @@ coherent_batch_split_kernel(const BatchJob *jobs, int n_jobs,
     if (it >= n_items) break;
     const BatchJob &J = jobs[s_job];
     const long long local = it - J.item0;
-    coherent_split_cta<ROUGH>(J.a, J.k, (int)(local % J.n_chunks),
-                              (int)(local / J.n_chunks), smem_raw);
+    coherent_split_cta<ROUGH, true, FORM>(J.a, J.k,
+                                          (int)(local % J.n_chunks),
+                                          (int)(local / J.n_chunks), smem_raw);
   }
 }
 
-// The build of the batch kernel for a CTA size (512 only for smooth
-// facets, which the batch layout enforces).
+// The build of the batch kernel for a CTA size (512 only for smooth facets,
+// which the batch layout enforces) and the jobs' form.
 template <int ROUGH>
-static void *batch_split_fn(int threads) {
+static void *batch_split_fn(int threads, int form) {
   if constexpr (ROUGH == SS_ROUGH_NONE) {
-    if (threads > 256)
+    if (threads > 256) {
+      if (form == kFormPlain)
+        return reinterpret_cast<void *>(
+            coherent_batch_split_kernel<ROUGH, 512, kFormPlain>);
+      if (form == kFormBeam)
+        return reinterpret_cast<void *>(
+            coherent_batch_split_kernel<ROUGH, 512, kFormBeam>);
       return reinterpret_cast<void *>(
-          coherent_batch_split_kernel<ROUGH, 512>);
+          coherent_batch_split_kernel<ROUGH, 512, kFormAny>);
+    }
   }
-  return reinterpret_cast<void *>(coherent_batch_split_kernel<ROUGH, 256>);
+  return reinterpret_cast<void *>(
+      coherent_batch_split_kernel<ROUGH, 256, kFormAny>);
 }
 
-static void *batch_split_fn_kind(int rough_kind, int threads) {
+static void *batch_split_fn_kind(int rough_kind, int threads, int form) {
   switch (rough_kind) {
-    case SS_ROUGH_NONE: return batch_split_fn<SS_ROUGH_NONE>(threads);
+    case SS_ROUGH_NONE: return batch_split_fn<SS_ROUGH_NONE>(threads, form);
     case SS_ROUGH_GAUSS_FULL:
-      return batch_split_fn<SS_ROUGH_GAUSS_FULL>(threads);
+      return batch_split_fn<SS_ROUGH_GAUSS_FULL>(threads, form);
     case SS_ROUGH_GAUSS_AREA:
-      return batch_split_fn<SS_ROUGH_GAUSS_AREA>(threads);
-    default: return batch_split_fn<SS_ROUGH_EXP_AREA>(threads);
+      return batch_split_fn<SS_ROUGH_GAUSS_AREA>(threads, form);
+    default: return batch_split_fn<SS_ROUGH_EXP_AREA>(threads, form);
   }
+}
+
+int coherent_form(const CoArgs &a) {
+  if (a.taper || a.split || a.interp) return kFormAny;
+  return a.pat_kind == SS_PAT_ISOTROPIC ? kFormPlain : kFormBeam;
 }
 
 int coherent_batch_split_launch(const BatchJob *jobs, int n_jobs,
                                 long long n_items,
                                 unsigned long long *counter, int rough_kind,
-                                int threads, int ctas, size_t smem,
+                                int form, int threads, int ctas, size_t smem,
                                 cudaStream_t st) {
   // the dynamic shared-memory limit was raised at prepare time, so this
   // path holds only stream operations (it may run under graph capture)
-  void *fn = batch_split_fn_kind(rough_kind, threads);
+  void *fn = batch_split_fn_kind(rough_kind, threads, form);
   void *args[] = {(void *)&jobs, (void *)&n_jobs, (void *)&n_items,
                   (void *)&counter};
   return cuda_status(cudaLaunchKernel(fn, dim3(ctas), dim3(threads), args,
@@ -606,13 +640,14 @@ int coherent_batch_split_launch(const BatchJob *jobs, int n_jobs,
                      "batch split launch");
 }
 
-int batch_split_blocks_per_sm(int rough_kind, int threads, size_t smem) {
+int batch_split_blocks_per_sm(int rough_kind, int form, int threads,
+                              size_t smem) {
   // raise the kernel's dynamic shared-memory limit to the largest size any
   // prepared batch uses (never lowered: earlier batches stay launchable)
-  static size_t limit[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  const int r = (rough_kind & 3) * 2 + (threads > 256 ? 1 : 0);
+  static size_t limit[24] = {};
+  const int r = ((rough_kind & 3) * 2 + (threads > 256 ? 1 : 0)) * 3 + form;
   limit[r] = std::max(limit[r], smem);
-  void *fn = batch_split_fn_kind(rough_kind, threads);
+  void *fn = batch_split_fn_kind(rough_kind, threads, form);
   int n = 0;
   cudaError_t e = cudaFuncSetAttribute(
       fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit[r]);
@@ -655,18 +690,36 @@ int coherent_split_launch(CoArgs &a, const Plan &p, cudaStream_t st) {
                 (a.rough_kind ? (size_t)(a.n_terms + 1) * sizeof(float) : 0);
   cudaError_t e = cudaSuccess;
   switch (a.rough_kind) {
-#define SS_LAUNCH(R)                                                         \
-  case R:                                                                    \
-    e = cudaFuncSetAttribute(coherent_split_kernel<R>,                       \
-                             cudaFuncAttributeMaxDynamicSharedMemorySize,    \
-                             (int)smem);                                     \
-    if (e != cudaSuccess) return cuda_status(e, "coherent_split smem");      \
-    coherent_split_kernel<R><<<grid, p.threads, smem, st>>>(a, k);           \
-    break;
-    SS_LAUNCH(SS_ROUGH_NONE)
-    SS_LAUNCH(SS_ROUGH_GAUSS_FULL)
-    SS_LAUNCH(SS_ROUGH_GAUSS_AREA)
-    SS_LAUNCH(SS_ROUGH_EXP_AREA)
+#define SS_LAUNCH(R, P)                                                      \
+  e = cudaFuncSetAttribute(coherent_split_kernel<R, P>,                      \
+                           cudaFuncAttributeMaxDynamicSharedMemorySize,      \
+                           (int)smem);                                       \
+  if (e != cudaSuccess) return cuda_status(e, "coherent_split smem");        \
+  coherent_split_kernel<R, P><<<grid, p.threads, smem, st>>>(a, k);
+    case SS_ROUGH_NONE:
+      switch (coherent_form(a)) {
+        case kFormPlain: {
+          SS_LAUNCH(SS_ROUGH_NONE, kFormPlain)
+          break;
+        }
+        case kFormBeam: {
+          SS_LAUNCH(SS_ROUGH_NONE, kFormBeam)
+          break;
+        }
+        default: {
+          SS_LAUNCH(SS_ROUGH_NONE, kFormAny)
+        }
+      }
+      break;
+    case SS_ROUGH_GAUSS_FULL:
+      SS_LAUNCH(SS_ROUGH_GAUSS_FULL, kFormAny)
+      break;
+    case SS_ROUGH_GAUSS_AREA:
+      SS_LAUNCH(SS_ROUGH_GAUSS_AREA, kFormAny)
+      break;
+    case SS_ROUGH_EXP_AREA:
+      SS_LAUNCH(SS_ROUGH_EXP_AREA, kFormAny)
+      break;
 #undef SS_LAUNCH
     default:
       return SS_ERR_ARG;

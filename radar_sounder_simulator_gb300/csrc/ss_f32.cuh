@@ -46,6 +46,62 @@ __device__ __forceinline__ float sinc32(float x) {
   return __fdividef(sin_red(x), x);
 }
 
+// MUFU operations without the denormal-range fix-ups the plain intrinsics
+// carry (three instructions each), for lengths, cosines, ratios and reduced
+// angles, which are never denormal.
+__device__ __forceinline__ float rsq_n(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float rcp_n(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float sin_n(float x) {
+  float y;
+  asm("sin.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float cos_n(float x) {
+  float y;
+  asm("cos.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float exp2_n(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// sinc32 with those.
+__device__ __forceinline__ float sinc_n(float x) {
+  const float x2 = x * x;
+  if (x2 < 0.25f)
+    return __fmaf_rn(x2, __fmaf_rn(x2, __fmaf_rn(x2, __fmaf_rn(
+               x2, 2.7557319e-06f, -1.9841270e-04f), 8.3333333e-03f),
+               -1.6666667e-01f), 1.0f);
+  return sin_n(reduce_2pi(x)) * rcp_n(x);
+}
+
+// (re, im) into a bin of a shared-memory histogram by one 64-bit
+// compare-and-swap: two float atomics are two such loops of 32 bits.
+__device__ __forceinline__ void hist_add(float2 *h, float re, float im) {
+  unsigned long long *p = reinterpret_cast<unsigned long long *>(h);
+  unsigned long long old = *reinterpret_cast<volatile unsigned long long *>(p),
+                     was;
+  do {
+    was = old;
+    const float2 v =
+        make_float2(__int_as_float((int)was) + re,
+                    __int_as_float((int)(was >> 32)) + im);
+    old = atomicCAS(p, was,
+                    ((unsigned long long)(unsigned)__float_as_int(v.y) << 32) |
+                        (unsigned)__float_as_int(v.x));
+  } while (old != was);
+}
+
 __device__ __forceinline__ float dot3f(float ax, float ay, float az, float bx,
                                        float by, float bz) {
   return __fmaf_rn(az, bz, __fmaf_rn(ay, by, ax * bx));

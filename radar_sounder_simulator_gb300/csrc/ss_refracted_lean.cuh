@@ -285,7 +285,7 @@ __device__ __forceinline__ bool lean_path(
   }
   G.opl = df_make(opl_h, opl_l + dopl);
   G.valid = ok && res <= tol * tol;
-  G.att = exp2f(expo);
+  G.att = exp2_n(expo);
   // spreading: l_perp = n0 sum(s/n), l_par = n0 c0^2 sum(s / (n c^2)), flux
   // = n0 c0 / (nj c_last)
   const float cl = fmaxf(cout, 1e-9f);

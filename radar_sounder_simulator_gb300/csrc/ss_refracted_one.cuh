@@ -30,19 +30,6 @@
 
 namespace ss {
 
-// MUFU operations without the denormal-range fix-ups the plain intrinsics
-// carry, for lengths, cosines and their ratios (never denormal).
-__device__ __forceinline__ float rsq_n(float x) {
-  float y;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-__device__ __forceinline__ float rcp_n(float x) {
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
 // Root sigma of ar tan(theta) + bd tan(theta') = L, sin(theta') = r
 // sin(theta), by bracketed Newton (refraction.py:120-144): the rays the
 // short iteration below leaves unsettled.
@@ -352,7 +339,7 @@ __device__ __forceinline__ void one_path(const OnePlane &M, const OneLegs &k,
   const float cc1 = c1 * c1, cc2 = c2 * c2;
   G.spread = 4.0f * cc1 * cc2 *
              rcp_n(D * D * ((l1 + l2) * __fmaf_rn(l1, cc2, l2 * cc1)));
-  G.att = exp2f(__fmaf_rn(s1.hi, k.x1, s2.hi * k.x2));
+  G.att = exp2_n(__fmaf_rn(s1.hi, k.x1, s2.hi * k.x2));
 #pragma unroll
   for (int j = 0; j < 3; ++j) {
     G.rh[j] = y[j] * is2;

@@ -1055,7 +1055,8 @@ __device__ __forceinline__ bool pair_finish(
     facet_edges(f, f1, f2, gam);
     const float d1 = dot3a(rh, f1), d2 = dot3a(rh, f2);
     const float base = k.amp_pref_j * gam * cos_t * spread * G.att;
-    float amp = base * fa * sinc32(k.kj * d1) * sinc32(k.kj * d2);
+    float amp = ONE ? base * fa * sinc_n(k.kj * d1) * sinc_n(k.kj * d2)
+                    : base * fa * sinc32(k.kj * d1) * sinc32(k.kj * d2);
     if (!PLAIN && a.taper) {
       const float ct = fminf(fmaxf(cos_t, (float)kCMin), 1.0f);
       const float ct2 = ct * ct;
@@ -1122,7 +1123,12 @@ __device__ __forceinline__ bool pair_finish(
     float red = __fmaf_rn(-n2, 6.28318548202514648f, ph);  // exact
     red = __fmaf_rn(-n2, -1.74845553146951e-07f, red) + pl;
     float sn, cs;
-    __sincosf(red, &sn, &cs);
+    if (ONE) {
+      sn = sin_n(red);
+      cs = cos_n(red);
+    } else {
+      __sincosf(red, &sn, &cs);
+    }
     re = cr * sn - ci * cs;
     im = cr * cs + ci * sn;
     pwr = re * re + im * im;
@@ -1387,8 +1393,7 @@ __device__ __forceinline__ void refracted_split_cta(const RefArgs &a,
       }
       if (o.bin >= 0) {
         float2 *h = hist + (size_t)tt * a.n_seg + o.bin;
-        atomicAdd(&h->x, o.re);
-        if (a.coherent) atomicAdd(&h->y, o.im);
+        hist_add(h, o.re, o.im);
       } else {
         atomicAdd(&s_drop[tt], o.pwr);
       }
