@@ -2,26 +2,50 @@
 //
 // Same trace-block x facet-chunk decomposition and shared-memory histograms
 // as the surface kernel (ss_coherent.cu). Per (trace, target facet) pair the
-// refracted path is solved in float64 exactly as the reference program does:
-//   sequential: per crossed interface a 10-iteration two-point Snell solve
-//     on the mean plane anchors an affine facet lookup, then a 25-iteration
-//     solve on that facet's tangent plane (multilayer.py:352-406);
+// refracted path is solved in float64 to the reference program's result:
+//   sequential: per crossed interface a two-point Snell solve on the mean
+//     plane anchors an affine facet lookup, then a solve on that facet's
+//     tangent plane (multilayer.py:352-406);
 //   joint: the mean-plane chain anchors every lookup, then a damped Newton on
 //     2-D in-plane offsets with block-tridiagonal (Thomas) steps and step
 //     halving solves all crossings at once (multilayer.py:408-457,
 //     refraction_joint.py:249-322);
+// the solvers are ss_refracted_fp64.cuh and, with lookups and starts in
+// float32, ss_refracted_lean64.cuh;
 // followed by Fresnel transmission, ray-tube spreading, two-way attenuation,
 // antenna gain, the facet's sinc response at the local wavenumber,
 // roughness, diffuse channel and binning (multilayer.py:500-583).
 #include <algorithm>
 
 #include "ss_refracted_fp64.cuh"
+#include "ss_refracted_lean64.cuh"
+#include "ss_refracted_split.cuh"
 
 namespace ss {
 
-template <int NI>
+// Path of one pair. LEAN: up to four interfaces, `col` the facet's lookup
+// constants.
+template <int NI, bool LEAN>
+__device__ __forceinline__ void path64(const RefArgs &a, const Lean64Consts &k,
+                                       const float *col, const float *qf,
+                                       const double *p, const double *q,
+                                       Path64 &P) {
+  if constexpr (NI == 0) {
+    if constexpr (LEAN) {
+      path_lean_chain64(a, k, col, p, q, P);
+    } else {
+      path_sequential64(a, p, q, P);
+    }
+  } else {
+    if constexpr (LEAN)
+      if (lean_path64<NI>(a, k, col, qf, p, q, P)) return;
+    path_joint64<NI>(a, p, q, P);
+  }
+}
+
+template <int NI, bool LEAN>
 __global__ void __launch_bounds__(128)
-refracted_fp64_kernel(RefArgs a) {
+refracted_fp64_kernel(RefArgs a, const __grid_constant__ Lean64Consts k) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double2 *hist = reinterpret_cast<double2 *>(smem_raw);
   double *lgam = reinterpret_cast<double *>(hist + (size_t)a.tb * a.n_seg);
@@ -66,21 +90,30 @@ refracted_fp64_kernel(RefArgs a) {
   const int nj = a.leg_last;  // final medium (multilayer.py:506)
   const double n0 = a.n_leg[0], njn = a.n_leg[nj];
   const double kj = a.k0 * njn, kj_pi = kj / kPi, amp_pref = kj / kTwoPi;
+  // fast-time bin u = opl bA - bB; the reference's own chain decides a pair
+  // within 1e-8 bins of an edge (the two differ by ~1e-11 bins)
+  const double bA = 2.0 / (a.c * a.dt), bB = a.t0 / a.dt;
   for (int i = s_rng[0] + tid; i < s_rng[1]; i += blockDim.x) {
-    const double q[3] = {(double)a.F.cx[i], (double)a.F.cy[i],
-                         (double)a.F.cz[i]};
+    const float qf[3] = {a.F.cx[i], a.F.cy[i], a.F.cz[i]};
+    const double q[3] = {(double)qf[0], (double)qf[1], (double)qf[2]};
+    float col[LEAN ? kLeanMax * kOnePerIface : 1];
+    if constexpr (LEAN) {
+      if constexpr (NI > 0) {
+        lean_facet<NI>(k.pl, qf, col, 1);
+      } else {
+        for (int j = 0; j < a.ni; ++j)
+          lean_facet<1>(k.pl + j, qf, col + j * kOnePerIface, 1);
+      }
+    }
     const double fn[3] = {(double)a.F.nx[i], (double)a.F.ny[i],
                           (double)a.F.nz[i]};
     const double fa = a.F.area[i];
     for (int tt = 0; tt < nt; ++tt) {
       if (i < s_lo[tt] || i >= s_hi[tt]) continue;
       Path64 P;
-      if (NI == 0)
-        path_sequential64(a, s_p[tt], q, P);
-      else
-        path_joint64<NI == 0 ? 1 : NI>(a, s_p[tt], q, P);
+      path64<NI, LEAN>(a, k, col, qf, s_p[tt], q, P);
       // final leg (medium j): crossing -> facet
-      double d[3] = {P.cur[0] - q[0], P.cur[1] - q[1], P.cur[2] - q[2]};
+      const double *d = P.d;
       double s_j, inv;
       sqrt_inv64(fmax(dot3v(d, d), 1e-60), s_j, inv);
       const double rh[3] = {d[0] * inv, d[1] * inv, d[2] * inv};
@@ -155,8 +188,12 @@ refracted_fp64_kernel(RefArgs a) {
         im = 0.0;
         pwr = re;
       }
-      const double twtt = __ddiv_rn(__dmul_rn(2.0, opl), a.c);
-      const double fb = floor(__ddiv_rn(__dsub_rn(twtt, a.t0), a.dt));
+      const double u = fma(opl, bA, -bB);
+      double fb = floor(u);
+      if (fabs(u - rint(u)) < 1e-8) {
+        const double twtt = __ddiv_rn(__dmul_rn(2.0, opl), a.c);
+        fb = floor(__ddiv_rn(__dsub_rn(twtt, a.t0), a.dt));
+      }
       const bool ok = P.valid && fb >= 0.0 && fb < (double)a.n_samples;
       if (ok) {
         int b = (int)fb;
@@ -272,16 +309,38 @@ static size_t refracted_scratch(const ss_refracted_opts *o, int T, int N) {
   return hist + drop + defer_mask_bytes(o, T, N);
 }
 
-template <int NI>
+template <int NI, bool LEAN>
 static int launch_fp64(RefArgs &a, const Plan &p, size_t smem,
                        cudaStream_t st) {
   cudaError_t e = cudaFuncSetAttribute(
-      refracted_fp64_kernel<NI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-      (int)smem);
+      refracted_fp64_kernel<NI, LEAN>,
+      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return cuda_status(e, "refracted_fp64 smem");
+  Lean64Consts k{};
+  if (LEAN) {
+    const RefSplitConsts c = split_consts(a);
+    for (int i = 0; i < kLeanMax; ++i) k.pl[i] = c.pl[i];
+    k.legs = c.lean;
+  }
   dim3 grid(p.n_chunks, p.n_groups);
-  refracted_fp64_kernel<NI><<<grid, p.threads, smem, st>>>(a);
+  refracted_fp64_kernel<NI, LEAN><<<grid, p.threads, smem, st>>>(a, k);
   return cuda_status(cudaGetLastError(), "refracted_fp64 launch");
+}
+
+// The float32 lookups and starts serve up to four interfaces whose cell
+// indices are exact in float32; a joint call also needs the step budget that
+// lean_path64 relies on, real permittivities that are the indices' squares
+// (its transmission) and smooth crossings.
+static bool lean_fp64(const RefArgs &a) {
+  if (a.ni > kLeanMax) return false;
+  for (int i = 0; i < a.ni; ++i)
+    if (a.ifc[i].ny >= (1 << 22) || a.ifc[i].nx >= (1 << 22)) return false;
+  if (!a.joint) return true;
+  for (int i = 0; i <= a.ni; ++i)
+    if (!(std::fabs(a.n_leg[i] * a.n_leg[i] - a.eps_leg[i]) <=
+          1e-13 * a.eps_leg[i]))
+      return false;
+  return a.n_newton >= 4 && a.n_backtrack >= 1 && !a.rough_cross;
 }
 
 }  // namespace ss
@@ -454,19 +513,29 @@ extern "C" int ss_refracted_fwd(const ss_refracted_opts *opts,
   if (opts->precision == SS_PREC_FP64) {
     const size_t smem = (size_t)p.tb * a.n_seg * 16 +
                         (a.rough_kind ? (a.n_terms + 1) * sizeof(double) : 0);
-    if (!a.joint) s = launch_fp64<0>(a, p, smem, st);
-    else switch (a.ni) {
-      case 1: s = launch_fp64<1>(a, p, smem, st); break;
-      case 2: s = launch_fp64<2>(a, p, smem, st); break;
-      case 3: s = launch_fp64<3>(a, p, smem, st); break;
-      case 4: s = launch_fp64<4>(a, p, smem, st); break;
-      case 5: s = launch_fp64<5>(a, p, smem, st); break;
-      case 6: s = launch_fp64<6>(a, p, smem, st); break;
-      case 7: s = launch_fp64<7>(a, p, smem, st); break;
-      case 8: s = launch_fp64<8>(a, p, smem, st); break;
+    const bool lean = lean_fp64(a);
+    if (!a.joint) {
+      s = lean ? launch_fp64<0, true>(a, p, smem, st)
+               : launch_fp64<0, false>(a, p, smem, st);
+    } else if (lean) {
+      switch (a.ni) {
+        case 1: s = launch_fp64<1, true>(a, p, smem, st); break;
+        case 2: s = launch_fp64<2, true>(a, p, smem, st); break;
+        case 3: s = launch_fp64<3, true>(a, p, smem, st); break;
+        default: s = launch_fp64<4, true>(a, p, smem, st); break;
+      }
+    } else switch (a.ni) {
+      case 1: s = launch_fp64<1, false>(a, p, smem, st); break;
+      case 2: s = launch_fp64<2, false>(a, p, smem, st); break;
+      case 3: s = launch_fp64<3, false>(a, p, smem, st); break;
+      case 4: s = launch_fp64<4, false>(a, p, smem, st); break;
+      case 5: s = launch_fp64<5, false>(a, p, smem, st); break;
+      case 6: s = launch_fp64<6, false>(a, p, smem, st); break;
+      case 7: s = launch_fp64<7, false>(a, p, smem, st); break;
+      case 8: s = launch_fp64<8, false>(a, p, smem, st); break;
       // deeper stacks (firn runs cross tens of layers): one instantiation
       // whose joint-solve arrays hold SS_MAX_IFACE interfaces
-      default: s = launch_fp64<kDeepNI>(a, p, smem, st); break;
+      default: s = launch_fp64<kDeepNI, false>(a, p, smem, st); break;
     }
   } else {
     s = refracted_split_launch(a, p, st);

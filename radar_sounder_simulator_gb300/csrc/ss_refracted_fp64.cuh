@@ -376,25 +376,40 @@ static __device__ __noinline__ void joint64(
 
 // Path result shared by both solvers (multilayer.py `path` returns).
 struct Path64 {
-  double cur[3], xf[3];
+  double d[3], xf[3];  // last crossing - q; first crossing
   bool valid;
   double opl, loss_db, sum_par, sum_perp, tau2, c0, c_last;
 };
 
-static __device__ __noinline__ void path_sequential64(const RefArgs &a, const double *p,
-                                  const double *q, Path64 &P) {
+// The plane of each lookup of the sequential chain: anchored by the float64
+// mean-plane crossing.
+struct Cell64 {
+  __device__ __forceinline__ void operator()(const RefArgs &a, int i,
+                                             const double *cur,
+                                             const double *q, double *pt,
+                                             double *nr) const {
+    const ss_interface &I = a.ifc[i];
+    Snell64 R;
+    snell64(cur, q, I.mean_point, I.mean_normal, a.n_leg[i], a.n_leg[i + 1],
+            10, R, true);
+    lookup64(I, R.x, pt, nr);
+  }
+};
+
+template <typename Cell>
+static __device__ __forceinline__ void path_chain64(const RefArgs &a,
+                                                    const double *p,
+                                                    const double *q, Path64 &P,
+                                                    Cell cell) {
   double cur[3] = {p[0], p[1], p[2]};
   P.valid = true;
   P.opl = P.loss_db = P.sum_par = P.sum_perp = 0.0;
   P.tau2 = 1.0;
   P.c0 = P.c_last = 1.0;
   for (int i = 0; i < a.ni; ++i) {
-    const ss_interface &I = a.ifc[i];
     const double n1 = a.n_leg[i], n2 = a.n_leg[i + 1];
-    Snell64 R1;
-    snell64(cur, q, I.mean_point, I.mean_normal, n1, n2, 10, R1, true);
     double pt[3], nr[3];
-    lookup64(I, R1.x, pt, nr);
+    cell(a, i, cur, q, pt, nr);
     const double inn = rsqrt(dot3v(nr, nr));
     for (int j = 0; j < 3; ++j) nr[j] *= inn;
     Snell64 R;
@@ -420,7 +435,14 @@ static __device__ __noinline__ void path_sequential64(const RefArgs &a, const do
     P.c_last = fmax(R.c2, kCMin);
     for (int j = 0; j < 3; ++j) cur[j] = R.x[j];
   }
-  for (int j = 0; j < 3; ++j) P.cur[j] = cur[j];
+  for (int j = 0; j < 3; ++j) P.d[j] = cur[j] - q[j];
+}
+
+static __device__ __noinline__ void path_sequential64(const RefArgs &a,
+                                                      const double *p,
+                                                      const double *q,
+                                                      Path64 &P) {
+  path_chain64(a, p, q, P, Cell64());
 }
 
 template <int NI>
@@ -475,7 +497,7 @@ static __device__ __noinline__ void path_joint64(const RefArgs &a, const double 
   P.c0 = c_surf;
   P.c_last = fmax(cout_[ni - 1], kCMin);
   for (int j = 0; j < 3; ++j) {
-    P.cur[j] = X[ni - 1][j];
+    P.d[j] = X[ni - 1][j] - q[j];
     P.xf[j] = X[0][j];
   }
 }
@@ -491,9 +513,8 @@ static __device__ __noinline__ double full_opl64(const RefArgs &a, const double 
     path_sequential64(a, p, q, P);
   else
     path_joint64<NI == 0 ? 1 : NI>(a, p, q, P);
-  double d[3] = {P.cur[0] - q[0], P.cur[1] - q[1], P.cur[2] - q[2]};
   valid = P.valid;
-  return P.opl + a.n_leg[a.leg_last] * sqrt(dot3v(d, d));
+  return P.opl + a.n_leg[a.leg_last] * sqrt(dot3v(P.d, P.d));
 }
 
 }  // namespace ss

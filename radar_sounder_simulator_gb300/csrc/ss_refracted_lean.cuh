@@ -55,17 +55,89 @@ __device__ __forceinline__ void lean_facet(const OnePlane *M, const float *q,
   }
 }
 
-// One pair; false when it needs the fix-up (a cell decision near a boundary,
-// a steep plane, an unsettled solve).
+// Newton step (tx, ty) of the crossings of a polyline with unit leg
+// directions d, weights w = n / length and gradient (f0, f1), which it uses
+// up: blocks of the Hessian from p = B^T d_i and r = B^T d_(i+1), block
+// elimination and back substitution. Returns the step's size (a NaN stays
+// in it).
 template <int NI>
-__device__ __forceinline__ bool lean_path(
-    const OnePlane *M, const LeanLegs &k, const ss_interface *ifc, int k_pad,
-    int n_newton, const float *col, int stride, const float *q, float4 A,
-    float2 Bp, float tol, PairGeo &G) {
-  const float P[3] = {A.x - q[0], A.y - q[1], A.z - q[2]};
+__device__ __forceinline__ float lean_step(
+    const float (&w)[NI + 1], const float (&d)[NI + 1][3],
+    const float (&sx)[NI], const float (&sy)[NI], float (&f0)[NI],
+    float (&f1)[NI], float (&tx)[NI], float (&ty)[NI]) {
+  float a00[NI], a01[NI], a11[NI], C[NI][4];
+#pragma unroll
+  for (int i = 0; i < NI; ++i) {
+    const float p0 = __fmaf_rn(sx[i], d[i][2], d[i][0]);
+    const float p1 = __fmaf_rn(sy[i], d[i][2], d[i][1]);
+    const float r0 = __fmaf_rn(sx[i], d[i + 1][2], d[i + 1][0]);
+    const float r1 = __fmaf_rn(sy[i], d[i + 1][2], d[i + 1][1]);
+    const float ws = w[i] + w[i + 1];
+    const float wp0 = w[i] * p0, wp1 = w[i] * p1;
+    const float wr0 = w[i + 1] * r0, wr1 = w[i + 1] * r1;
+    const float g01 = sx[i] * sy[i];
+    a00[i] = __fmaf_rn(-wp0, p0, __fmaf_rn(-wr0, r0,
+                 ws * __fmaf_rn(sx[i], sx[i], 1.0f)));
+    a01[i] = __fmaf_rn(-wp0, p1, __fmaf_rn(-wr0, r1, ws * g01));
+    a11[i] = __fmaf_rn(-wp1, p1, __fmaf_rn(-wr1, r1,
+                 ws * __fmaf_rn(sy[i], sy[i], 1.0f)));
+    if (i + 1 < NI) {
+      // C_i = -w B_i^T (I - d d^T) B_(i+1) of the shared leg
+      const float m0 = __fmaf_rn(sx[i + 1], d[i + 1][2], d[i + 1][0]);
+      const float m1 = __fmaf_rn(sy[i + 1], d[i + 1][2], d[i + 1][1]);
+      const float ww = w[i + 1];
+      C[i][0] = __fmaf_rn(wr0, m0, -ww * __fmaf_rn(sx[i], sx[i + 1], 1.0f));
+      C[i][1] = __fmaf_rn(wr0, m1, -ww * (sx[i] * sy[i + 1]));
+      C[i][2] = __fmaf_rn(wr1, m0, -ww * (sy[i] * sx[i + 1]));
+      C[i][3] = __fmaf_rn(wr1, m1, -ww * __fmaf_rn(sy[i], sy[i + 1], 1.0f));
+    }
+    if (i > 0) {
+      // minus C^T A^-1 of the interface above (a: its inverse)
+      const float u00 = C[i - 1][0] * a00[i - 1] + C[i - 1][2] * a01[i - 1];
+      const float u01 = C[i - 1][0] * a01[i - 1] + C[i - 1][2] * a11[i - 1];
+      const float u10 = C[i - 1][1] * a00[i - 1] + C[i - 1][3] * a01[i - 1];
+      const float u11 = C[i - 1][1] * a01[i - 1] + C[i - 1][3] * a11[i - 1];
+      a00[i] -= u00 * C[i - 1][0] + u01 * C[i - 1][2];
+      a01[i] -= u00 * C[i - 1][1] + u01 * C[i - 1][3];
+      a11[i] -= u10 * C[i - 1][1] + u11 * C[i - 1][3];
+      f0[i] -= u00 * f0[i - 1] + u01 * f1[i - 1];
+      f1[i] -= u10 * f0[i - 1] + u11 * f1[i - 1];
+    }
+    const float id = rcp_n(a00[i] * a11[i] - a01[i] * a01[i]);
+    const float b00 = a11[i] * id, b11 = a00[i] * id;
+    a01[i] = -a01[i] * id;
+    a00[i] = b00;
+    a11[i] = b11;
+  }
+  float big = 0.0f;
+#pragma unroll
+  for (int i = NI - 1; i >= 0; --i) {
+    float g0 = f0[i], g1 = f1[i];
+    if (i + 1 < NI) {
+      const float t0 = tx[i + 1 < NI ? i + 1 : i];
+      const float t1 = ty[i + 1 < NI ? i + 1 : i];
+      g0 -= C[i][0] * t0 + C[i][1] * t1;
+      g1 -= C[i][2] * t0 + C[i][3] * t1;
+    }
+    tx[i] = a00[i] * g0 + a01[i] * g1;
+    ty[i] = a01[i] * g0 + a11[i] * g1;
+    big += fabsf(tx[i]) + fabsf(ty[i]);
+  }
+  return big;
+}
+
+// Table cells of a pair, the looked-up planes' slopes over q and the
+// crossings (X, Y, Z) from q; P = p - q. False when the pair needs the
+// fix-up (a cell decision near a boundary, a steep plane, an unsettled
+// solve).
+template <int NI>
+__device__ __forceinline__ bool lean_solve(
+    const OnePlane *M, const LeanLegs &k, const ss_interface *ifc,
+    int n_newton, const float *col, int stride, const float *q,
+    const float (&P)[3], int (&cell)[NI], float (&sx)[NI], float (&sy)[NI],
+    float (&X)[NI], float (&Y)[NI], float (&Z)[NI]) {
+  float c[NI];
   // mean-plane chain: cells and the crossings that start the solve
-  int cell[NI];
-  float X[NI], Y[NI], sx[NI], sy[NI], c[NI];
   {
     float v[3] = {P[0], P[1], P[2]};
     bool safe = true;
@@ -95,7 +167,6 @@ __device__ __forceinline__ bool lean_path(
     }
     if (!safe) return false;
   }
-  float Z[NI];
   auto heights = [&]() {
 #pragma unroll
     for (int i = 0; i < NI; ++i)
@@ -123,9 +194,8 @@ __device__ __forceinline__ bool lean_path(
       d[s][1] = dy * il;
       d[s][2] = dz * il;
     }
-    // gradient F_i = B_i^T (n_(i+1) d_(i+1) - n_i d_i); blocks of the
-    // Hessian from p = B^T d_i and r = B^T d_(i+1); forward elimination
-    float a00[NI], a01[NI], a11[NI], C[NI][4], f0[NI], f1[NI];
+    // gradient F_i = B_i^T (n_(i+1) d_(i+1) - n_i d_i)
+    float f0[NI], f1[NI], tx[NI], ty[NI];
 #pragma unroll
     for (int i = 0; i < NI; ++i) {
       const float p0 = __fmaf_rn(sx[i], d[i][2], d[i][0]);
@@ -134,64 +204,33 @@ __device__ __forceinline__ bool lean_path(
       const float r1 = __fmaf_rn(sy[i], d[i + 1][2], d[i + 1][1]);
       f0[i] = __fmaf_rn(k.n[i + 1], r0, -k.n[i] * p0);
       f1[i] = __fmaf_rn(k.n[i + 1], r1, -k.n[i] * p1);
-      const float ws = w[i] + w[i + 1];
-      const float wp0 = w[i] * p0, wp1 = w[i] * p1;
-      const float wr0 = w[i + 1] * r0, wr1 = w[i + 1] * r1;
-      const float g01 = sx[i] * sy[i];
-      a00[i] = __fmaf_rn(-wp0, p0, __fmaf_rn(-wr0, r0,
-                   ws * __fmaf_rn(sx[i], sx[i], 1.0f)));
-      a01[i] = __fmaf_rn(-wp0, p1, __fmaf_rn(-wr0, r1, ws * g01));
-      a11[i] = __fmaf_rn(-wp1, p1, __fmaf_rn(-wr1, r1,
-                   ws * __fmaf_rn(sy[i], sy[i], 1.0f)));
-      if (i + 1 < NI) {
-        // C_i = -w B_i^T (I - d d^T) B_(i+1) of the shared leg
-        const float m0 = __fmaf_rn(sx[i + 1], d[i + 1][2], d[i + 1][0]);
-        const float m1 = __fmaf_rn(sy[i + 1], d[i + 1][2], d[i + 1][1]);
-        const float ww = w[i + 1];
-        C[i][0] = __fmaf_rn(wr0, m0, -ww * __fmaf_rn(sx[i], sx[i + 1], 1.0f));
-        C[i][1] = __fmaf_rn(wr0, m1, -ww * (sx[i] * sy[i + 1]));
-        C[i][2] = __fmaf_rn(wr1, m0, -ww * (sy[i] * sx[i + 1]));
-        C[i][3] = __fmaf_rn(wr1, m1, -ww * __fmaf_rn(sy[i], sy[i + 1], 1.0f));
-      }
-      if (i > 0) {
-        // minus C^T A^-1 of the interface above (a: its inverse)
-        const float u00 = C[i - 1][0] * a00[i - 1] + C[i - 1][2] * a01[i - 1];
-        const float u01 = C[i - 1][0] * a01[i - 1] + C[i - 1][2] * a11[i - 1];
-        const float u10 = C[i - 1][1] * a00[i - 1] + C[i - 1][3] * a01[i - 1];
-        const float u11 = C[i - 1][1] * a01[i - 1] + C[i - 1][3] * a11[i - 1];
-        a00[i] -= u00 * C[i - 1][0] + u01 * C[i - 1][2];
-        a01[i] -= u00 * C[i - 1][1] + u01 * C[i - 1][3];
-        a11[i] -= u10 * C[i - 1][1] + u11 * C[i - 1][3];
-        f0[i] -= u00 * f0[i - 1] + u01 * f1[i - 1];
-        f1[i] -= u10 * f0[i - 1] + u11 * f1[i - 1];
-      }
-      const float id = rcp_n(a00[i] * a11[i] - a01[i] * a01[i]);
-      const float b00 = a11[i] * id, b11 = a00[i] * id;
-      a01[i] = -a01[i] * id;
-      a00[i] = b00;
-      a11[i] = b11;
     }
-    // back substitution: X -= A^-1 (F + C step); a NaN stays in `big`
-    float big = 0.0f, t0 = 0.0f, t1 = 0.0f;
+    const float big = lean_step<NI>(w, d, sx, sy, f0, f1, tx, ty);
 #pragma unroll
-    for (int i = NI - 1; i >= 0; --i) {
-      float g0 = f0[i], g1 = f1[i];
-      if (i + 1 < NI) {
-        g0 -= C[i][0] * t0 + C[i][1] * t1;
-        g1 -= C[i][2] * t0 + C[i][3] * t1;
-      }
-      t0 = a00[i] * g0 + a01[i] * g1;
-      t1 = a01[i] * g0 + a11[i] * g1;
-      X[i] -= t0;
-      Y[i] -= t1;
-      big += fabsf(t0) + fabsf(t1);
+    for (int i = 0; i < NI; ++i) {
+      X[i] -= tx[i];
+      Y[i] -= ty[i];
     }
     heights();
     // a step of 1e-5 of the path leaves ~1e-10 of it in the crossing, whose
     // effect on the optical path is second order
     settled = big < 1e-5f * reach;
   }
-  if (!settled) return false;
+  return settled;
+}
+
+// One pair; false when it needs the fix-up.
+template <int NI>
+__device__ __forceinline__ bool lean_path(
+    const OnePlane *M, const LeanLegs &k, const ss_interface *ifc, int k_pad,
+    int n_newton, const float *col, int stride, const float *q, float4 A,
+    float2 Bp, float tol, PairGeo &G) {
+  const float P[3] = {A.x - q[0], A.y - q[1], A.z - q[2]};
+  int cell[NI];
+  float X[NI], Y[NI], Z[NI], sx[NI], sy[NI];
+  if (!lean_solve<NI>(M, k, ifc, n_newton, col, stride, q, P, cell, sx, sy, X,
+                      Y, Z))
+    return false;
   // legs as double-floats, cosines, residual, heights off the planes
   float uh[3], ul[3], is = 0.0f;
   float opl_h = 0.0f, opl_l = 0.0f, dopl = 0.0f, expo = 0.0f, perp = 0.0f;
