@@ -10,11 +10,21 @@
 // Everything is float32 like the reference. The bin is an integer decision
 // that must match the reference's float32 chain
 //   r = sqrt((dx^2 + dy^2) + dz^2), tw = (2 r) / c, u = (tw - t0) / dt
-// bit for bit, with each operation rounded to nearest. The kernel evaluates
-// it first as r A - B from a MUFU reciprocal square root, with an error
-// bound; only pairs whose fast value lies within that bound of an integer
-// re-run the exactly rounded chain (__fsqrt_rn / __fdiv_rn), so the bins
-// equal the reference's while the common case costs a few instructions.
+// bit for bit, with each operation rounded to nearest. The root is a MUFU
+// reciprocal root's with one Newton step, which is the rounded one unless
+// the exact root lies within 2^-14 ulp of a midpoint between two floats: the
+// exact remainder S - r^2 tells, and those pairs (one in 16,000) take
+// __fsqrt_rn. A quotient by a call constant b is x RN(1/b) with the
+// reciprocal's low part (Brisebarre and Muller, "Correctly rounded
+// multiplication by arbitrary precision constants"), right to an ulp, and one
+// remainder step with RN(1/b), which rounds it correctly (Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000
+// processor"; b's mantissa not all ones). So the chain is the reference's
+// with no branch but the rare one, where a bounded estimate sent one pair in
+// sixty -- 40% of the warps -- through the full root and quotients.
+//
+// The arithmetic runs on two traces at a time (packed float32: one issue
+// slot for two results, rounded alike).
 //
 // Work decomposition: the grid is (facet chunks) x (trace blocks of TB
 // traces). Each thread takes one facet at a time and evaluates it against
@@ -24,10 +34,17 @@
 // piling onto one address. Dropped power stays in registers (each step s
 // maps a thread to one fixed trace). Per-CTA histograms go to scratch and a
 // second kernel sums the chunks in a fixed order in float64.
+//
+// Bound by instruction issue (63 per pair, 68% of the slots at 32 warps per
+// SM, a third of them the histogram's compare-and-swap loops): 512^2 facets x
+// 1024 traces 855 -> 640 us.
 #include <algorithm>
+#include <cstdint>
+#include <cstring>
 
 #include "ss_chunksum.cuh"
 #include "ss_f32.cuh"
+#include "ss_f32x2.cuh"
 #include "ss_internal.cuh"
 
 namespace ss {
@@ -37,7 +54,9 @@ struct IncArgs {
   const double *pos, *uct, *pv;
   int pv_len, T, N, n_samples, n_seg, stride, split;
   float t0, dt, c;  // window scalars rounded to float32
-  float A, B, bandA;  // 2/(c dt), t0/dt, 1e-6 A of those float32 scalars
+  // quotients by c / 2 and dt: the divisors negated, reciprocals, low parts
+  float nhc, ndt, zc, zcl, zd, zdl;
+  float mid;  // bound of the midpoint test, in r ulp(r); negative: exact chain
   int pat_kind, pat_n;
   const double *pa, *pb;
   int n_chunks;
@@ -45,15 +64,31 @@ struct IncArgs {
   double *part_drop;  // (n_chunks, T) partial dropped power
 };
 
-// Exactly rounded float32 bin chain of the reference (geometry.py:6-24).
-__device__ __forceinline__ float bin_exact(float S, const IncArgs &a) {
+// Exactly rounded float32 bin coordinate of the reference (geometry.py:6-24).
+static __device__ __noinline__ float bin_exact(float S, float c, float t0,
+                                               float dt) {
   const float r = __fsqrt_rn(S);
-  const float tw = __fdiv_rn(__fmul_rn(2.0f, r), a.c);
-  return floorf(__fdiv_rn(__fsub_rn(tw, a.t0), a.dt));
+  const float tw = __fdiv_rn(__fmul_rn(2.0f, r), c);
+  return __fdiv_rn(__fsub_rn(tw, t0), dt);
+}
+
+// RN(x / b): z = RN(1/b), zl its low part, nb = -b.
+__device__ __forceinline__ float2 div_const2(float2 x, float z, float zl,
+                                             float nb) {
+  const float2 q = fma2(x, pk1(z), mul2(x, pk1(zl)));
+  return fma2(fma2(q, pk1(nb), x), pk1(z), q);
+}
+
+// CTA size: two 512-thread CTAs (64 registers) hold 32 warps per SM where
+// 256-thread ones (73 registers, and room for three 64 KB histograms) hold
+// 24; an antenna pattern needs twice the registers.
+template <bool PAT>
+constexpr int inc_threads() {
+  return PAT ? 256 : 512;
 }
 
 template <int TB, bool PAT>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(inc_threads<PAT>(), PAT ? 1 : 2)
 incoherent_kernel(IncArgs a) {
   extern __shared__ __align__(16) float hist[];  // (TB, stride)
   __shared__ float4 s_p[TB], s_u[TB];
@@ -99,17 +134,26 @@ incoherent_kernel(IncArgs a) {
   __syncthreads();
 
   // step s always pairs this thread with trace (lane + s) mod TB: its
-  // position, histogram row and dropped sum live in registers
-  float px[TB], py[TB], pz[TB], drop[TB];
+  // position, histogram row and dropped sum live in registers, two steps to a
+  // packed pair (TB = 1: the second half repeats the first and is not used)
+  constexpr int H = (TB + 1) / 2;
+  float2 px[H], py[H], pz[H];
+  float drop[TB];
   int hoff[TB];
 #pragma unroll
   for (int s = 0; s < TB; ++s) {
     const int tt = (lane + s) & (TB - 1);
     const float4 P = s_p[tt];
-    px[s] = P.x;
-    py[s] = P.y;
-    pz[s] = P.z;
-    hoff[s] = tt * a.stride;
+    if (s & 1) {
+      px[s / 2].y = P.x;
+      py[s / 2].y = P.y;
+      pz[s / 2].y = P.z;
+    } else {
+      px[s / 2] = pk1(P.x);
+      py[s / 2] = pk1(P.y);
+      pz[s / 2] = pk1(P.z);
+    }
+    hoff[s] = tt * a.stride - 0x4B000000;
     drop[s] = 0.f;
   }
 
@@ -119,55 +163,72 @@ incoherent_kernel(IncArgs a) {
   const float nsf = (float)a.n_samples;
 
   for (int i = i0 + tid; i < i1; i += blockDim.x) {
-    const float cx = a.cx[i], cy = a.cy[i], cz = a.cz[i];
-    const float nx = a.nx[i], ny = a.ny[i], nz = a.nz[i];
-    const float ar = a.area[i];
+    const float2 cx = pk1(a.cx[i]), cy = pk1(a.cy[i]), cz = pk1(a.cz[i]);
+    const float2 nx = pk1(a.nx[i]), ny = pk1(a.ny[i]), nz = pk1(a.nz[i]);
+    const float2 ar = pk1(a.area[i]);
 #pragma unroll
-    for (int s = 0; s < TB; ++s) {
-      const float dx = __fsub_rn(px[s], cx);
-      const float dy = __fsub_rn(py[s], cy);
-      const float dz = __fsub_rn(pz[s], cz);
-      const float S = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx),
-                                          __fmul_rn(dy, dy)),
-                                __fmul_rn(dz, dz));
-      const float y = rsqrtf(S);  // 1/r
+    for (int h = 0; h < H; ++h) {
+      const float2 dx = sub2(px[h], cx);
+      const float2 dy = sub2(py[h], cy);
+      const float2 dz = sub2(pz[h], cz);
+      // (scalar sums: the compiler fuses a packed sum of packed products)
+      const float2 x2 = mul2(dx, dx), yy = mul2(dy, dy), z2 = mul2(dz, dz);
+      const float2 S = pk(__fadd_rn(__fadd_rn(x2.x, yy.x), z2.x),
+                          __fadd_rn(__fadd_rn(x2.y, yy.y), z2.y));
+      const float2 y = pk(rsq_n(S.x), rsq_n(S.y));  // 1/r
       // power (A cos)^2 / r^4 = (A (d . n))^2 / r^6
-      const float q = ar * dot3f(dx, dy, dz, nx, ny, nz);
-      const float y2 = y * y;
-      float pw = (q * q) * (y2 * y2 * y2);
-      if (PAT) {
-        // departure direction antenna -> facet (incoherent.py:45)
-        const int tt = (lane + s) & (TB - 1);
-        const float g = gain32(a.pat_kind, a.pat_n, pa_len, s_pat, s_pv[tt],
-                               -dx * y, -dy * y, -dz * y);
-        const float g2 = g * g;
-        pw *= g2 * g2;
+      const float2 q =
+          mul2(ar, fma2(dz, nz, fma2(dy, ny, mul2(dx, nx))));
+      const float2 y2 = mul2(y, y);
+      float2 pw = mul2(mul2(q, q), mul2(mul2(y2, y2), y2));
+      // the reference's bin coordinate
+      const float2 g = mul2(S, y), hy = mul2(y, pk1(0.5f));
+      const float2 r = fma2(pk(__fmaf_rn(-g.x, g.x, S.x),
+                               __fmaf_rn(-g.y, g.y, S.y)), hy, g);
+      const float ex = __fmaf_rn(-r.x, r.x, S.x),
+                  ey = __fmaf_rn(-r.y, r.y, S.y);
+      // 2^k of the binade just below r: a power of two's lower neighbour is
+      // half an ulp away
+      const float2 rb = mul2(r, pk1(0.99999994f));
+      const float2 k2 = pk(__int_as_float(__float_as_int(rb.x) & 0x7f800000),
+                           __int_as_float(__float_as_int(rb.y) & 0x7f800000));
+      const float2 lim = mul2(mul2(r, k2), pk1(a.mid));
+      const float2 tw = div_const2(r, a.zc, a.zcl, a.nhc);
+      float2 u = div_const2(sub2(tw, pk1(a.t0)), a.zd, a.zdl, a.ndt);
+      if (fabsf(ex) > lim.x || fabsf(ey) > lim.y) {
+        u.x = bin_exact(S.x, a.c, a.t0, a.dt);
+        u.y = bin_exact(S.y, a.c, a.t0, a.dt);
       }
-      // fast bin u ~ r A - B (A = 2/(c dt), B = t0/dt) and its error bound
-      // |uf - u| <= 4.8e-7 r A + 2.4e-7 |u| (rsqrt 2 ulp, A, B and the
-      // roundings of both chains); the band doubles that. A pair the bound
-      // cannot settle takes the exact chain; a band of half a bin or more
-      // sends every pair there.
-      const float rf = S * y;
-      const float uf = __fmaf_rn(rf, a.A, -a.B);
-      float fb = floorf(uf);
-      const float fr = uf - fb;
-      const float band =
-          __fmaf_rn(a.bandA, rf, __fmaf_rn(7e-7f, fabsf(uf), 1e-6f));
-      if (fminf(fr, 1.0f - fr) < band) fb = bin_exact(S, a);
-      if (fb >= 0.0f && fb < nsf) {
-        int seg = (int)fb;
-        if (a.split) {
-          const float4 U = s_u[(lane + s) & (TB - 1)];
-          // (c - p) . u_ct, rounded like the reference's sum
-          const float sd = __fadd_rn(__fadd_rn(__fmul_rn(-dx, U.x),
-                                               __fmul_rn(-dy, U.y)),
-                                     __fmul_rn(-dz, U.z));
-          if (sd > 0.0f) seg += a.n_samples;
+#pragma unroll
+      for (int j = 0; j < 2 && 2 * h + j < TB; ++j) {
+        const int s = 2 * h + j;
+        const float us = j ? u.y : u.x;
+        float p = j ? pw.y : pw.x;
+        const float dxs = j ? dx.y : dx.x, dys = j ? dy.y : dy.x,
+                    dzs = j ? dz.y : dz.x, ys = j ? y.y : y.x;
+        if (PAT) {
+          // departure direction antenna -> facet (incoherent.py:45)
+          const int tt = (lane + s) & (TB - 1);
+          const float gn = gain32(a.pat_kind, a.pat_n, pa_len, s_pat, s_pv[tt],
+                                  -dxs * ys, -dys * ys, -dzs * ys);
+          const float g2 = gn * gn;
+          p *= g2 * g2;
         }
-        atomicAdd(&hist[hoff[s] + seg], pw);
-      } else {
-        drop[s] += pw;
+        if (us >= 0.0f && us < nsf) {
+          // floor: 2^23 + u rounded down has it in the low mantissa bits
+          int seg = __float_as_int(__fadd_rd(us, 8388608.0f));
+          if (a.split) {
+            const float4 U = s_u[(lane + s) & (TB - 1)];
+            // (c - p) . u_ct, rounded like the reference's sum
+            const float sd = __fadd_rn(__fadd_rn(__fmul_rn(-dxs, U.x),
+                                                 __fmul_rn(-dys, U.y)),
+                                       __fmul_rn(-dzs, U.z));
+            if (sd > 0.0f) seg += a.n_samples;
+          }
+          atomicAdd(&hist[hoff[s] + seg], p);
+        } else {
+          drop[s] += p;
+        }
       }
     }
   }
@@ -237,13 +298,24 @@ int inc_plan(const ss_incoherent_opts *o, int T, int N, IncPlan *p) {
   p->tb = tb;
   p->smem = tb * row;
   p->n_groups = (T + tb - 1) / tb;
-  // about eight CTAs per SM in total, each chunk at least 2048 facets and
-  // enough pairs to amortise zeroing and writing its histograms
-  const int sms = sm_count();
-  const long target = 8L * sms;
-  long nc = (target + p->n_groups - 1) / p->n_groups;
-  nc = std::min(nc, std::max(1L, (long)N / 2048));
-  nc = std::min(nc, std::max(1L, (long)N * tb / (4L * n_seg)));
+  // two to four waves of two CTAs per SM, the count that fills its last wave
+  // best (a wave half full costs a full one); each chunk at least 2048 facets
+  // and enough pairs to amortise zeroing and writing its histograms
+  const long slots = 2L * sm_count();
+  const long most = std::max(1L, std::min((long)N / 2048,
+                                          (long)N * tb / (4L * n_seg)));
+  long nc = 1;
+  double best = 0.0;
+  for (long w = 2; w <= 4; ++w) {
+    const long k = std::max(1L, std::min(most, w * slots / p->n_groups));
+    const long items = k * p->n_groups;
+    const double fill =
+        (double)items / (double)((items + slots - 1) / slots * slots);
+    if (fill > best + 1e-9) {
+      best = fill;
+      nc = k;
+    }
+  }
   p->n_chunks = (int)std::max(1L, nc);
   return SS_OK;
 }
@@ -255,7 +327,7 @@ int inc_launch_t(const IncArgs &a, const IncPlan &p, cudaStream_t st) {
       (int)p.smem);
   if (e != cudaSuccess) return cuda_status(e, "incoherent smem");
   dim3 grid(p.n_chunks, p.n_groups);
-  incoherent_kernel<TB, PAT><<<grid, 256, p.smem, st>>>(a);
+  incoherent_kernel<TB, PAT><<<grid, inc_threads<PAT>(), p.smem, st>>>(a);
   return cuda_status(cudaGetLastError(), "incoherent launch");
 }
 
@@ -348,9 +420,25 @@ extern "C" int ss_incoherent_fwd(const ss_incoherent_opts *opts,
   a.t0 = (float)opts->t0;
   a.dt = (float)opts->dt;
   a.c = (float)opts->c;
-  a.A = (float)(2.0 / ((double)a.c * (double)a.dt));
-  a.B = (float)((double)a.t0 / (double)a.dt);
-  a.bandA = 1e-6f * a.A;
+  const float hc = 0.5f * a.c;
+  a.nhc = -hc;
+  a.ndt = -a.dt;
+  const double ic = 1.0 / (double)hc, id = 1.0 / (double)a.dt;
+  a.zc = (float)ic;
+  a.zcl = (float)(ic - (double)a.zc);
+  a.zd = (float)id;
+  a.zdl = (float)(id - (double)a.zd);
+  // The fast chain's quotients want divisors whose mantissa is not all ones
+  // and whose products stay clear of float32's range ends; any other call
+  // takes the exact chain throughout.
+  const auto plain = [](float b) {
+    uint32_t bits;
+    std::memcpy(&bits, &b, 4);
+    return b > 1e-15f && b < 1e15f && (bits & 0x7fffffu) != 0x7fffffu;
+  };
+  a.mid = plain(hc) && plain(a.dt)
+              ? (float)((1.0 - 1.0 / 16384) / 8388608.0)
+              : -1.0f;
   a.pat_kind = kind;
   a.pat_n = pattern ? pattern->n : 0;
   a.pa = pattern ? pattern->pa : nullptr;
