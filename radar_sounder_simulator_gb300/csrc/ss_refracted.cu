@@ -93,6 +93,9 @@ refracted_fp64_kernel(RefArgs a, const __grid_constant__ Lean64Consts k) {
   // fast-time bin u = opl bA - bB; the reference's own chain decides a pair
   // within 1e-8 bins of an edge (the two differ by ~1e-11 bins)
   const double bA = 2.0 / (a.c * a.dt), bB = a.t0 / a.dt;
+  // a warp's lanes take the traces in rotated order, so that neighbouring
+  // facets' bins are not one bin's updates in turn (ss_refracted_split.cuh)
+  const int rot = (tid & 31) % max(nt, 1);
   for (int i = s_rng[0] + tid; i < s_rng[1]; i += blockDim.x) {
     const float qf[3] = {a.F.cx[i], a.F.cy[i], a.F.cz[i]};
     const double q[3] = {(double)qf[0], (double)qf[1], (double)qf[2]};
@@ -108,7 +111,8 @@ refracted_fp64_kernel(RefArgs a, const __grid_constant__ Lean64Consts k) {
     const double fn[3] = {(double)a.F.nx[i], (double)a.F.ny[i],
                           (double)a.F.nz[i]};
     const double fa = a.F.area[i];
-    for (int tt = 0; tt < nt; ++tt) {
+    for (int st = 0; st < nt; ++st) {
+      const int tt = st + rot < nt ? st + rot : st + rot - nt;
       if (i < s_lo[tt] || i >= s_hi[tt]) continue;
       Path64 P;
       path64<NI, LEAN>(a, k, col, qf, s_p[tt], q, P);
