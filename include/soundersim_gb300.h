@@ -374,6 +374,14 @@ int ss_facets_from_vertices(const double *vertices, int32_t H, int32_t W,
 int ss_speckle_phasors_keyed(const int64_t *keys, int64_t n, uint64_t base,
                              float *out, void *stream);
 
+/* Facet records for the kernels: (n, 3) / (n) float64 device arrays gathered
+ * by order (n) and rounded to float32 into soa (13, n): center, normal, e1,
+ * e2, area. */
+int ss_stage_facets(const double *centers, const double *normals,
+                    const double *e1, const double *e2, const double *areas,
+                    const int64_t *order, int32_t n, float *soa,
+                    void *stream);
+
 /* Facet centres moved `offset` metres along local ellipsoidal up
  * (layered.py:38-53 offset_facets; normals, areas and edges unchanged). */
 int ss_offset_centers(const double *centers, int64_t n, const ss_frame *frame,

@@ -278,6 +278,8 @@ SIGNATURES = {
                                            C.c_void_p]),
     "ss_offset_centers": (C.c_int, [C.c_void_p, C.c_int64, C.POINTER(Frame),
                                     C.c_double, C.c_void_p, C.c_void_p]),
+    "ss_stage_facets": (C.c_int, [C.c_void_p] * 6 + [C.c_int32, C.c_void_p,
+                                                     C.c_void_p]),
     "ss_trace_products_scratch_bytes": (C.c_size_t, [C.c_int32, C.c_int32]),
     "ss_trace_products": (C.c_int, [C.POINTER(TraceProductsOpts), C.c_void_p,
                                     C.c_int32, C.c_void_p, C.c_int32,

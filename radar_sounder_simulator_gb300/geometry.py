@@ -36,8 +36,16 @@ class CullPlan(NamedTuple):
     n_win: int             # blocks per window
 
 
+def along_track(pos, cen):
+    """Projections of facets and traces on the first->last track axis."""
+    d = pos[-1, :2] - pos[0, :2]
+    nrm = np.linalg.norm(d)
+    axis = d / nrm if nrm > 0 else np.array([1.0, 0.0])
+    return cen[:, :2] @ axis, pos[:, :2] @ axis
+
+
 def cull_plan(positions, centers, *, t0, dt, n_samples, c, block_size,
-              target_pairs, window_cull=True, device=None):
+              target_pairs, window_cull=True, device=None, projected=None):
     """Order + windows as coherent.py:284-296 / multilayer.py:684-697.
 
     With a CUDA ``device`` the sort and the window searches run there: the
@@ -45,22 +53,19 @@ def cull_plan(positions, centers, *, t0, dt, n_samples, c, block_size,
     them, uploaded, stably sorted (equal keys keep their index order, -0.0
     counts as +0.0, as in NumPy's comparison) and searched on the device;
     the permutation stays there as an int64 tensor and only the per-trace
-    window offsets come back."""
+    window offsets come back. ``projected``: ``along_track``'s two results and
+    the facets' as a device tensor, from a caller that has them there."""
     pos = np.asarray(positions, np.float64)
     cen = np.asarray(centers, np.float64)
     n = len(cen)
     bs = min(block_size or auto_block_size(len(pos), target_pairs), n)
     n_blocks = -(-n // bs)
-    d = pos[-1, :2] - pos[0, :2]
-    nrm = np.linalg.norm(d)
-    axis = d / nrm if nrm > 0 else np.array([1.0, 0.0])
-    s_f = cen[:, :2] @ axis
+    s_f, s_t, keys = projected or (*along_track(pos, cen), None)
     if device is not None and torch.device(device).type == "cuda":
-        return _cull_plan_device(s_f + 0.0, pos[:, :2] @ axis, bs, n_blocks,
-                                 t0, dt, n_samples, c, window_cull, device)
+        return _cull_plan_device(s_f, s_t, keys, bs, n_blocks, t0, dt,
+                                 n_samples, c, window_cull, device)
     order = np.argsort(s_f, kind="stable")
     s_sorted = s_f[order]
-    s_t = pos[:, :2] @ axis
     if not window_cull:
         return CullPlan(order, bs, n_blocks, np.zeros(len(pos), np.int32),
                         int(n_blocks))
@@ -74,14 +79,18 @@ def cull_plan(positions, centers, *, t0, dt, n_samples, c, block_size,
     return CullPlan(order, bs, n_blocks, off, n_win)
 
 
-def _cull_plan_device(s_f, s_t, bs, n_blocks, t0, dt, n_samples, c,
+def _cull_plan_device(s_f, s_t, keys, bs, n_blocks, t0, dt, n_samples, c,
                       window_cull, device):
-    keys = torch.from_numpy(s_f).to(device)
+    if keys is None:
+        keys = torch.from_numpy(s_f + 0.0).to(device)
     s_sorted, order = torch.sort(keys, stable=True)
-    if not window_cull:
+    reach = window_reach_m(t0, dt, n_samples, c)
+    # where every trace reaches the whole scene the searches would return 0
+    # and n: nothing to wait for
+    if not window_cull or (s_f.min() >= (s_t - reach).max() and
+                           s_f.max() <= (s_t + reach).min()):
         return CullPlan(order, bs, n_blocks, np.zeros(len(s_t), np.int32),
                         int(n_blocks))
-    reach = window_reach_m(t0, dt, n_samples, c)
     lo_v = torch.from_numpy(s_t - reach).to(device)
     hi_v = torch.from_numpy(s_t + reach).to(device)
     lo = torch.searchsorted(s_sorted, lo_v, right=False)
