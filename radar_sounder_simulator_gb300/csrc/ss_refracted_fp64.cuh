@@ -198,32 +198,32 @@ __device__ __forceinline__ void joint_geom(const double (&B)[NI][3][2],
 }
 
 // Newton step delta at geometry G: the block-tridiagonal system assembled
-// and solved (block Thomas, refraction_joint.py:218-246) in float32. Only
-// the residual needs float64: a step with a float32 matrix leaves ~1e-7 of
-// itself, less than the quadratic remainder of the first steps and less
-// than an ulp of the last. With orthonormal in-plane bases the 2x2 blocks
+// and solved (block Thomas, refraction_joint.py:218-246) in F. Only the
+// residual needs float64 on the way to a root: a step with a float32 matrix
+// leaves ~1e-7 of itself, less than the quadratic remainder of the first
+// steps and less than an ulp of the last. With orthonormal in-plane bases the 2x2 blocks
 // follow from the projections, B_i^T (n/s)(I - d d^T) B_j = (n/s)(B_i^T B_j
 // - (B_i^T d)(B_j^T d)^T). Returns max |delta|.
-template <int NI>
-__device__ __forceinline__ float joint_step(const JointGeom<NI> &G,
-                                            const float (&BB)[NI][2][2],
-                                            const double *nm,
-                                            float (&delta)[NI][2], int ni) {
-  const float mu = 1.8e-12f;  // Levenberg shift, float64 eps^0.75
-  float w[NI + 1], Cm[NI][2][2], dinv[NI][2][2], y[NI][2];
-  for (int k = 0; k <= ni; ++k) w[k] = (float)(nm[k] * G.is[k]);
+template <int NI, class F>
+__device__ __forceinline__ F joint_step(const JointGeom<NI> &G,
+                                        const F (&BB)[NI][2][2],
+                                        const double *nm, F (&delta)[NI][2],
+                                        int ni) {
+  const F mu = (F)1.8189894035458565e-12;  // Levenberg shift, eps^0.75
+  F w[NI + 1], Cm[NI][2][2], dinv[NI][2][2], y[NI][2];
+  for (int k = 0; k <= ni; ++k) w[k] = (F)(nm[k] * G.is[k]);
   for (int i = 0; i < ni; ++i) {
-    const float p[2] = {(float)G.pin[i][0], (float)G.pin[i][1]};
-    const float q[2] = {(float)G.pout[i][0], (float)G.pout[i][1]};
-    float M[2][2], rhs[2] = {-(float)G.f[i][0], -(float)G.f[i][1]};
+    const F p[2] = {(F)G.pin[i][0], (F)G.pin[i][1]};
+    const F q[2] = {(F)G.pout[i][0], (F)G.pout[i][1]};
+    F M[2][2], rhs[2] = {-(F)G.f[i][0], -(F)G.f[i][1]};
     for (int r = 0; r < 2; ++r)
       for (int c = 0; c < 2; ++c) {
-        const float e = r == c ? 1.0f : 0.0f;
+        const F e = r == c ? (F)1 : (F)0;
         M[r][c] = w[i] * (e - p[r] * p[c]) + w[i + 1] * (e - q[r] * q[c]) +
                   e * mu;
       }
     if (i > 0) {
-      float cpt[2][2];  // C_{i-1}^T dinv_{i-1}
+      F cpt[2][2];  // C_{i-1}^T dinv_{i-1}
       for (int r = 0; r < 2; ++r)
         for (int c = 0; c < 2; ++c)
           cpt[r][c] = Cm[i - 1][0][r] * dinv[i - 1][0][c] +
@@ -235,9 +235,9 @@ __device__ __forceinline__ float joint_step(const JointGeom<NI> &G,
         rhs[r] -= cpt[r][0] * y[i - 1][0] + cpt[r][1] * y[i - 1][1];
       }
     }
-    float det = M[0][0] * M[1][1] - M[0][1] * M[1][0];
-    if (fabsf(det) < 1e-30f) det = 1e-30f;
-    const float id = 1.0f / det;
+    F det = M[0][0] * M[1][1] - M[0][1] * M[1][0];
+    if (fabs(det) < (F)1e-30) det = (F)1e-30;
+    const F id = (F)1 / det;
     dinv[i][0][0] = M[1][1] * id;
     dinv[i][0][1] = -M[0][1] * id;
     dinv[i][1][0] = -M[1][0] * id;
@@ -245,32 +245,34 @@ __device__ __forceinline__ float joint_step(const JointGeom<NI> &G,
     y[i][0] = rhs[0];
     y[i][1] = rhs[1];
     if (i + 1 < ni) {
-      const float pn[2] = {(float)G.pin[i + 1][0], (float)G.pin[i + 1][1]};
+      const F pn[2] = {(F)G.pin[i + 1][0], (F)G.pin[i + 1][1]};
       for (int r = 0; r < 2; ++r)
         for (int c = 0; c < 2; ++c)
           Cm[i][r][c] = -w[i + 1] * (BB[i][r][c] - q[r] * pn[c]);
     }
   }
-  float dmax = 0.0f;
+  F dmax = (F)0;
   for (int i = ni - 1; i >= 0; --i) {
-    float rr[2] = {y[i][0], y[i][1]};
+    F rr[2] = {y[i][0], y[i][1]};
     if (i < ni - 1)
       for (int r = 0; r < 2; ++r)
         rr[r] -= Cm[i][r][0] * delta[i + 1][0] + Cm[i][r][1] * delta[i + 1][1];
     for (int r = 0; r < 2; ++r) {
       delta[i][r] = dinv[i][r][0] * rr[0] + dinv[i][r][1] * rr[1];
-      dmax = fmaxf(dmax, fabsf(delta[i][r]));
+      dmax = fmax(dmax, fabs(delta[i][r]));
     }
   }
   return dmax;
 }
 
-template <int NI>
-static __device__ __noinline__ void joint64(
+// One solve with step matrices in F; false when the step budget (or the
+// halving) ran out before the steps became rounding.
+template <int NI, class F>
+static __device__ __noinline__ bool joint_solve64(
     const double *p, const double *q, const double (&O)[NI][3],
     const double (&Nn)[NI][3], const double *nm, int n_newton,
     int n_backtrack, double (&X)[NI][3], double (&cinc)[NI],
-    double (&cout_)[NI], double (&S)[NI + 1], bool &valid, int ni = NI) {
+    double (&cout_)[NI], double (&S)[NI + 1], bool &valid, int ni) {
   // the path scale as a power of two: scaling rounds nothing
   const float pq[3] = {(float)(p[0] - q[0]), (float)(p[1] - q[1]),
                        (float)(p[2] - q[2])};
@@ -307,18 +309,19 @@ static __device__ __noinline__ void joint64(
       ab[i][c] = B[i][0][c] * y[0] + B[i][1][c] * y[1] + B[i][2][c] * y[2];
   }
   for (int j = 0; j < 3; ++j) D[ni][j] = (q[j] - O[ni - 1][j]) * inv;
-  float BB[NI][2][2];  // B_i^T B_{i+1}
+  F BB[NI][2][2];  // B_i^T B_{i+1}
   for (int i = 0; i + 1 < ni; ++i)
     for (int r = 0; r < 2; ++r)
       for (int c = 0; c < 2; ++c)
-        BB[i][r][c] = (float)(B[i][0][r] * B[i + 1][0][c] +
+        BB[i][r][c] = (F)(B[i][0][r] * B[i + 1][0][c] +
                               B[i][1][r] * B[i + 1][1][c] +
                               B[i][2][r] * B[i + 1][2][c]);
   JointGeom<NI> G;
   joint_geom<NI>(B, D, nm, ab, G, ni);
-  for (int it = 0; it < n_newton; ++it) {
-    float delta[NI][2];
-    const float dmax = joint_step<NI>(G, BB, nm, delta, ni);
+  bool done = false;
+  for (int it = 0; it < n_newton && !done; ++it) {
+    F delta[NI][2];
+    const F dmax = joint_step<NI, F>(G, BB, nm, delta, ni);
     // step halving on |F|^2; the accepted candidate's geometry is the next
     // iteration's
     const double m0 = G.m;
@@ -334,7 +337,7 @@ static __device__ __noinline__ void joint64(
       joint_geom<NI>(B, D, nm, ab, G, ni);
       // below 1e-9 of the path scale the residual is rounding: the step
       // itself is the correction
-      if (G.m < m0 || (dmax < 1e-9f && isfinite(G.m))) {
+      if (G.m < m0 || (dmax < (F)1e-9 && isfinite(G.m))) {
         moved = true;
         break;
       }
@@ -345,7 +348,7 @@ static __device__ __noinline__ void joint64(
       joint_geom<NI>(B, D, nm, ab, G, ni);
       break;
     }
-    if (dmax < 1e-9f) break;  // the remaining error is below rounding
+    done = dmax < (F)1e-9;  // the remaining error is below rounding
   }
   // crossings, legs and validity (refraction_joint.py:143-176): with
   // orthonormal bases the in-plane parts are the projections
@@ -372,6 +375,23 @@ static __device__ __noinline__ void joint64(
     fin = fin && isfinite(X[i][0]) && isfinite(X[i][1]) && isfinite(X[i][2]);
   }
   valid = (residual <= 1e-18) && isfinite(residual) && fin && sides && !evan;
+  return done;
+}
+
+// The joint solve (refraction_joint.py:249-322). A pair that the budget
+// leaves short of its root is judged by the residual it stopped at, which a
+// float32 matrix would leave elsewhere: those (none, as a rule) repeat the
+// reference's float64 steps.
+template <int NI>
+static __device__ __forceinline__ void joint64(
+    const double *p, const double *q, const double (&O)[NI][3],
+    const double (&Nn)[NI][3], const double *nm, int n_newton,
+    int n_backtrack, double (&X)[NI][3], double (&cinc)[NI],
+    double (&cout_)[NI], double (&S)[NI + 1], bool &valid, int ni = NI) {
+  if (!joint_solve64<NI, float>(p, q, O, Nn, nm, n_newton, n_backtrack, X,
+                                cinc, cout_, S, valid, ni))
+    joint_solve64<NI, double>(p, q, O, Nn, nm, n_newton, n_backtrack, X, cinc,
+                              cout_, S, valid, ni);
 }
 
 // Path result shared by both solvers (multilayer.py `path` returns).
