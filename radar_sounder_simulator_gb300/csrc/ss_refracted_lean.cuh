@@ -130,7 +130,7 @@ __device__ __forceinline__ float lean_step(
 // crossings (X, Y, Z) from q; P = p - q. False when the pair needs the
 // fix-up (a cell decision near a boundary, a steep plane, an unsettled
 // solve).
-template <int NI>
+template <int NI, int SOLVE = kLookup>
 __device__ __forceinline__ bool lean_solve(
     const OnePlane *M, const LeanLegs &k, const ss_interface *ifc,
     int n_newton, const float *col, int stride, const float *q,
@@ -150,8 +150,8 @@ __device__ __forceinline__ bool lean_solve(
       f.ri[1] = fc[2 * stride];
       f.rf[0] = fc[3 * stride];
       f.rf[1] = fc[4 * stride];
-      safe = one_cell(M[i], f, v, ifc[i].ny, ifc[i].nx, 1.0f + 0.5f * i,
-                      cell[i], v) && safe;
+      safe = one_cell<SOLVE>(M[i], f, v, ifc[i].ny, ifc[i].nx, 1.0f + 0.5f * i,
+                             cell[i], v) && safe;
       // the looked-up plane as a height field over q, and the crossing moved
       // vertically onto it
       float o[3], t[3];

@@ -5,7 +5,8 @@
 // count of float64 operations. Two parts of the path need none:
 //   * the mean-plane chain only picks table cells. The float32 chain of the
 //     split form (ss_refracted_one.cuh) picks the same ones except within a
-//     guard band of a cell boundary, where the float64 chain decides;
+//     guard band of a cell boundary and for flat rays (beyond 49 degrees on
+//     the rarer side), where the float64 chain decides;
 //   * Newton's method for the joint crossings forgets its start. The float32
 //     solve of ss_refracted_lean.cuh ends ~1e-7 from the root; from there
 //     each step with a float64 residual and a float32 matrix gains ~6 digits,
@@ -56,7 +57,7 @@ static __device__ __forceinline__ bool lean_path64(
     float X[NI], Y[NI], Z[NI];
     // two steps fewer than the float64 form has: a pair that settles (a last
     // step of 1e-5) is then one that form converges too
-    if (!lean_solve<NI>(k.pl, k.legs, a.ifc, a.n_newton - 2, col, 1, qf, Pf,
+    if (!lean_solve<NI, kLookup64>(k.pl, k.legs, a.ifc, a.n_newton - 2, col, 1, qf, Pf,
                         cell, sf, tf, X, Y, Z))
       return false;
 #pragma unroll
@@ -137,6 +138,8 @@ static __device__ __forceinline__ bool lean_path64(
     if (!(u1 * u2 > 0.0)) return false;
     cinc[i] = fabs(u1);
     cout_[i] = fabs(u2);
+    // near grazing the reference's start may be short of its root
+    if (fmin(cinc[i], cout_[i]) < 0.15) return false;
     if (a.n_leg[i] * a.n_leg[i] * (1.0 - u1 * u1) >
         a.n_leg[i + 1] * a.n_leg[i + 1])
       return false;
@@ -195,7 +198,7 @@ __device__ __forceinline__ bool lean_cell64(const RefArgs &a,
                       (float)(cur[2] - q[2])};
   int cell;
   float v[3], o[3], t[3];
-  if (!one_cell(k.pl[i], f, V, a.ifc[i].ny, a.ifc[i].nx, 1.0f + 0.5f * i,
+  if (!one_cell<kLookup64>(k.pl[i], f, V, a.ifc[i].ny, a.ifc[i].nx, 1.0f + 0.5f * i,
                 cell, v))
     return false;
   load_plane(k.pl[i].vec, a.ifc[i].table, cell, o, t);

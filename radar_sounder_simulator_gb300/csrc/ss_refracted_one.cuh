@@ -56,9 +56,22 @@ static __device__ __noinline__ float sigma_bracketed(float ar, float bd,
   return sig;
 }
 
+// The reference's lookup solve stops after ten iterations (multilayer.py:
+// 352-406), which reach the root for every sigma below 0.8 but leave some
+// flat rays short of it (0.04% of those at 0.8-0.9, 1% at 0.98; a float64
+// model over random heights, offsets and index ratios) and so pick other
+// cells. The float64 form's lookups (kLookup64) leave every ray past kFlatRay
+// to its float64 solve, which repeats those iterations; the split form takes
+// the root (platforms 30-240 m over a kilometre of rough facets: 1e-6 to
+// 2e-5 of the oracle, where the ten float32 iterations were no closer).
+constexpr float kFlatRay = 0.75f;
+enum { kOnFacet = 0, kLookup = 1, kLookup64 = 2 };
+
 // Fraction of the way from q's foot to p's foot at which the refracted ray
 // meets the plane: heights a of p and b of q over it, feet L apart (iL =
-// 1/L), r = n_rare / n_dense, `up` when p is on the rare side.
+// 1/L), r = n_rare / n_dense, `up` when p is on the rare side. kLookup64: NaN
+// for a flat ray.
+template <int SOLVE>
 __device__ __forceinline__ float cross_frac(float a, float b, float L,
                                             float L2, float iL, float r,
                                             float k2, float k4, bool up) {
@@ -85,8 +98,13 @@ __device__ __forceinline__ float cross_frac(float a, float b, float L,
     sig -= d;
     // remaining error ~1.5 tan^2-weighted d^2: below 1.5e-7 of sigma
     settled = d * d * q1 <= 1e-7f * sig * sig;
+    // q1 = 1 / (1 - sigma^2)
+    if (SOLVE == kLookup64)
+      settled = settled && q1 < 1.0f / (1.0f - kFlatRay * kFlatRay);
     if (settled) break;
   }
+  if (SOLVE == kLookup64)
+    return (settled ? off : __int_as_float(0x7fc00000)) * iL;
   if (!settled) {
     const float s = sigma_bracketed(ar, bd, L, r), v = r * s;
     off = up ? bd * v * rsqrtf(fmaxf((1.0f - v) * (1.0f + v), 1e-30f))
@@ -141,7 +159,9 @@ constexpr float kCellAbs = 5e-6f, kCellRel = 3e-6f;
 
 // Cell of the mean-plane crossing of the ray from q + P to q, and that
 // crossing from q (v, which may be P); false when a coordinate is within the
-// guard band of a rounding boundary.
+// guard band of a rounding boundary or the ray is one for float64 (a NaN
+// crossing compares false).
+template <int SOLVE = kLookup>
 __device__ __forceinline__ bool one_cell(const OnePlane &M, const OneFacet &f,
                                          const float *P, int ny, int nx,
                                          float scale, int &cell, float *v) {
@@ -151,8 +171,9 @@ __device__ __forceinline__ bool one_cell(const OnePlane &M, const OneFacet &f,
   const float wz = __fmaf_rn(-vn, M.mn[2], P[2]);
   const float L2 = fmaxf(dot3f(wx, wy, wz, wx, wy, wz), 1e-20f);
   const float iL = rsq_n(L2);
-  const float g = cross_frac(fabsf(vn - f.b), fabsf(f.b), L2 * iL, L2, iL,
-                             M.r, M.k2, M.k4, M.up);
+  const float a = fabsf(vn - f.b), b = fabsf(f.b);
+  const float g =
+      cross_frac<SOLVE>(a, b, L2 * iL, L2, iL, M.r, M.k2, M.k4, M.up);
   const float fr = __fmaf_rn(g, __fmaf_rn(M.c[0], wx, M.c[2] * wy), f.rf[0]);
   const float fc = __fmaf_rn(g, __fmaf_rn(M.c[1], wx, M.c[3] * wy), f.rf[1]);
   const float kr = rintf(fr), kc = rintf(fc);
@@ -299,7 +320,8 @@ __device__ __forceinline__ void one_path(const OnePlane &M, const OneLegs &k,
       fmaxf(dot3f(w[0], w[1], w[2], w[0], w[1], w[2]), 1e-20f);
   const float iL = rsq_n(L2), L = L2 * iL;
   const float aa = fabsf(a), ab = fabsf(b);
-  const float fg = cross_frac(aa, ab, L, L2, iL, M.r, M.k2, M.k4, M.up);
+  const float fg =
+      cross_frac<kOnFacet>(aa, ab, L, L2, iL, M.r, M.k2, M.k4, M.up);
   // crossing from q; legs in double-float
   float y[3], uh[3], ul[3], is1, is2;
 #pragma unroll

@@ -106,6 +106,33 @@ def test_refracted_paths_match_oracle(T, ni, joint, opt, precision):
         _split_ok(got, ref)
 
 
+@pytest.mark.parametrize("eps", [[1.0, 3.15, 5.0], [2.0, 1.0, 3.0],
+                                 [1.0, 1.05, 1.1]])
+@pytest.mark.parametrize("ni,refraction", [(1, "sequential"), (1, "joint"),
+                                           (2, "sequential"), (2, "joint")])
+@pytest.mark.parametrize("alt", [50.0, 140.0])
+def test_flat_rays_match_oracle(alt, ni, refraction, eps):
+    """A platform 50 m over a scene a kilometre wide: rays near grazing and
+    the critical angle, where the reference's ten lookup iterations end short
+    of their root and pick other cells."""
+    from radar_sounder_simulator_gb300.multilayer import refracted_cluttergram
+    layers = [_layer(24, 29, 40.0, -30.0 * j, 8.0 if j == 0 else 2.4, 70 + j)
+              for j in range(ni)]
+    bed = _layer(20, 26, 41.0, -30.0 * ni - 30.0, 8.0, 90)
+    pos, uct = _track(3, alt, step=50.0)
+    args = (pos, uct, bed, layers, eps[:ni + 1], [0.0, 1.0, 1.0][:ni + 1])
+    kw = dict(mode="coherent", t0=0.0, dt=4e-8, n_samples=600, c=C,
+              gamma=0.2, k0=K0, refraction=refraction)
+    ref, _ = oref.refracted_cluttergram(*args, **kw)
+    for precision in ("fp64", "split"):
+        got, _ = refracted_cluttergram(*args, **kw, precision=precision,
+                                       out_dtype=np.complex128)
+        if precision == "fp64":
+            assert np.abs(got - ref).max() <= 1e-9 * np.abs(ref).max()
+        else:
+            assert field_errors(got, ref)["rel_l2"] <= 1e-4
+
+
 SURFACE = [
     dict(), dict(pattern=True), dict(taper_s=0.3, split_sides=True),
     dict(interp_bins=True), dict(pattern=True, interp_bins=True)]
