@@ -1596,20 +1596,21 @@ def fp32_peak_tflops(device, repeats=5, fp64=False, mufu=False):
     return best
 
 
-# FP32 FLOP the bed kernel executes per pair, from the full ncu capture of
-# `python bench.py --kernel-only bed` (profiles/refracted_split_bed_512sq_
-# 1024tr_full.md): (2 FFMA + FADD + FMUL) per cycle x clock x duration /
-# pairs. The canonical count above follows the reference's float64 solve;
-# this one is what the float32 pipe runs (fewer Newton steps, table seeds).
-EXECUTED_FP32_FLOP_PER_PAIR = {"bed_joint": 3151.0}
+# FP32 FLOP the bed kernel executes per pair: (2 FFMA + FADD + FMUL thread
+# instructions) / pairs of an ncu capture over 256 traces
+# (profiles/short_paths_ncu.md). The canonical count above follows the
+# reference's float64 solve at its fixed budgets; this one is what the float32
+# pipe runs (converged solves, table-free bases).
+EXECUTED_FP32_FLOP_PER_PAIR = {"bed_joint": 2056.0}
 
 
 def roofline(per_kernel_ms, pairs, peak_tflops, traffic=None):
     """Dominant launch sequence's position against the FP32 pipe."""
     i = int(np.argmax(per_kernel_ms))
     names = ["surface", "h1_seq", "h2_joint", "bed_joint"]
-    kernels = ["coherent_split_kernel", "refracted_split_kernel<0>",
-               "refracted_split_kernel<2>", "refracted_split_kernel<3>"]
+    kernels = ["coherent_split_kernel", "refracted_split_kernel<kOneNI>",
+               "refracted_split_kernel<lean_class(2)>",
+               "refracted_split_kernel<lean_class(3)>"]
     C, joint = LAYER_PATHS[i]
     fl = pair_flops(C, joint)
     achieved = pairs[i] * fl / (per_kernel_ms[i] * 1e-3) / 1e12
@@ -1620,8 +1621,8 @@ def roofline(per_kernel_ms, pairs, peak_tflops, traffic=None):
         executed = {"flop_per_pair": xf, "achieved": xa,
                     "frac": xa / peak_tflops,
                     "source": "ncu FFMA/FADD/FMUL counts of this kernel "
-                              "(profiles/refracted_split_bed_512sq_1024tr_"
-                              "full.md) x the pairs timed here"}
+                              "(profiles/short_paths_ncu.md) x the pairs "
+                              "timed here"}
     return {"bound": "fp32", "achieved": achieved, "peak": peak_tflops,
             "unit": "TFLOP/s", "frac": achieved / peak_tflops,
             "executed": executed,

@@ -334,7 +334,8 @@ static int launch_fp64(RefArgs &a, const Plan &p, size_t smem,
 // The float32 lookups and starts serve up to four interfaces whose cell
 // indices are exact in float32; a joint call also needs the step budget that
 // lean_path64 relies on, real permittivities that are the indices' squares
-// (its transmission) and smooth crossings.
+// (its transmission) and smooth crossings. 120x96 facets x 40 traces through
+// two interfaces: 2.02 ms without, 0.64 ms with.
 static bool lean_fp64(const RefArgs &a) {
   if (a.ni > kLeanMax) return false;
   for (int i = 0; i < a.ni; ++i)
