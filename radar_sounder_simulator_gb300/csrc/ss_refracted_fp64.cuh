@@ -92,7 +92,8 @@ static __device__ __noinline__ double sigma_budget64(double ar, double bd,
 // and a step below 1e-9 of sigma leaves less than an ulp, so the iteration
 // ends there. Flat rays repeat the reference's iteration: ten steps reach the
 // root for every sigma below 0.8, twenty-five below 0.999 (a float64 model
-// over random heights, offsets and index ratios). `x_only`: the crossing point alone (lookup anchors).
+// over random heights, offsets and index ratios). `x_only`: the crossing point
+// alone (lookup anchors).
 static __device__ __noinline__ void snell64(const double *p, const double *q,
                                             const double *o,
                                             const double *nrm, double n1,
