@@ -272,11 +272,15 @@ int coherent_plan(const ss_coherent_opts *o, int T, int N, Plan *p,
   tb = std::min(tb, T);
   p->threads = fp64 || rough ? 256 : 512;
   const long window = std::min<long>((long)o->n_win * o->block_size, N);
-  // a chunk gives every thread of its CTA a facet (256-thread CTAs at least
-  // one, 512-thread ones half of them); a call too small to cover the SMs
-  // takes smaller trace blocks until it does (64^2 facets x 32 traces of
-  // 512 bins ran on 32 of 152 SMs)
-  const int max_chunks = (int)std::max<long>(1, window / 256);
+  // a chunk holds at least 512 facets (109x71 facets x 454 traces: 99 us in
+  // one wave of 5 chunks, 107 us in three of 16); a call too small to cover
+  // the SMs that way takes chunks of 256 and smaller trace blocks until it
+  // does (64^2 facets x 32 traces of 512 bins ran on 32 of 152 SMs)
+  long least = 512;
+  if ((long)((T + tb - 1) / tb) * std::max<long>(1, window / least) <
+      2L * sm_count())
+    least = 256;
+  const int max_chunks = (int)std::max<long>(1, window / least);
   while (tb > (fp64 ? 1 : 2) &&
          (long)((T + tb - 1) / tb) * max_chunks < 2L * sm_count())
     tb = (tb + 1) / 2;
