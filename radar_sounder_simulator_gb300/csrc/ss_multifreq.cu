@@ -167,20 +167,22 @@ multifreq_split_kernel(MfArgs a, MfSplitConsts k) {
   const int t_base = blockIdx.y * kMfTB;
   const int nt = min(kMfTB, a.T - t_base);
   const int tid = threadIdx.x;
-  if (tid < kMfTB) {
-    const int t = min(t_base + tid, a.T - 1);
+  // (strided: a narrow band's CTA has fewer threads than either has entries)
+  for (int e = tid; e < kMfTB; e += blockDim.x) {
+    const int t = min(t_base + e, a.T - 1);
     for (int j = 0; j < 3; ++j) {
       const df v = df_from_double(a.pos[3 * t + j]);
-      s_ph[tid][j] = v.hi;
-      s_pl[tid][j] = v.lo;
+      s_ph[e][j] = v.hi;
+      s_pl[e][j] = v.lo;
     }
     int lo, hi;
     trace_window(a, t, lo, hi);
-    s_lo[tid] = tid < nt ? lo : a.N;
-    s_hi[tid] = tid < nt ? hi : 0;
+    s_lo[e] = e < nt ? lo : a.N;
+    s_hi[e] = e < nt ? hi : 0;
   }
-  if (ROUGH == SS_ROUGH_GAUSS_FULL && tid < SS_FAD_N)
-    s_fad[tid] = (float)a.fad.a[tid];
+  if (ROUGH == SS_ROUGH_GAUSS_FULL)
+    for (int j = tid; j < SS_FAD_N; j += blockDim.x)
+      s_fad[j] = (float)a.fad.a[j];
   if (ROUGH != SS_ROUGH_NONE) fill_inv_table(lg, a.n_terms, tid, blockDim.x);
   __syncthreads();
   if (tid == 0) {
