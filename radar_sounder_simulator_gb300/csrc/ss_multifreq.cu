@@ -56,12 +56,15 @@ struct MfArgs {
 // the 8 frequencies a float32 step may drift over. A CTA has as many threads
 // as its share of the band needs (768 frequencies: 2 x 48; at a fixed 128 a
 // quarter of the lanes idled, 0.39 -> 0.31 ms at 96 x 128 facets x 100
-// traces).
+// traces), a warp at least: the pairs of a tile take every thread there is
+// (100x100 facets x 9 traces of 16 frequencies: 256 us with two threads, 87
+// with 32; 100x100 x 100 of 128: 189, 168; 234 with 64).
 constexpr int kMfThreads = 128, kMfF = 16, kMfTB = 4, kMfP = 32;
 constexpr int kMfTB2 = kMfTB / 2;
 constexpr int kMfFBlock = kMfThreads / 2 * kMfF;
 
-// Threads of half a CTA for K frequencies cut into equal blocks.
+// Threads of half a CTA for K frequencies cut into equal blocks; a CTA's
+// threads past both halves take part in the tiles' pairs only.
 static int mf_half(int K) {
   const int blocks = (K + kMfFBlock - 1) / kMfFBlock;
   return ((K + blocks - 1) / blocks + kMfF - 1) / kMfF;
@@ -72,6 +75,7 @@ constexpr int kMf64F = 8;
 constexpr int kMf64TB = 2, kMf64P = 64;
 
 struct MfSplitConsts {
+  int half;  // threads of half a CTA
   float Rch, Rcl;   // 4 pi / c (rad per metre per hertz) as double-float
   float dfh, dfl;   // frequency step B / K
   float f1h, f1l;   // first frequency f0 - B/2 + B/(2K)
@@ -198,7 +202,7 @@ multifreq_split_kernel(MfArgs a, MfSplitConsts k) {
   __syncthreads();
 
   // this thread's first frequency index and its frequency / wavenumber
-  const int n_half = blockDim.x / 2, half = tid / n_half;
+  const int n_half = k.half, half = tid / n_half;
   const int kn = (blockIdx.z * n_half + tid - half * n_half) * kMfF;
   float fsh, fsl;
   {
@@ -315,7 +319,7 @@ multifreq_split_kernel(MfArgs a, MfSplitConsts k) {
       if (FULL) s_pd[e0] = pd;
     }
     __syncthreads();
-    if (kn >= a.K) continue;  // past the band's end
+    if (kn >= a.K || half > 1) continue;  // past the band's end
     // --- phase B: every thread, its traces' pairs, its frequencies ---
 #pragma unroll
     for (int tt = 0; tt < kMfTB2; ++tt) {
@@ -659,9 +663,15 @@ static int mf_plan(const ss_multifreq_opts *o, int T, int N, Plan *p) {
   const int fblk = (o->n_freq + kMfFBlock - 1) / kMfFBlock;
   const long window = std::min<long>((long)o->n_win * o->block_size, N);
   const int tile = f64 ? kMf64P : kMfP;
-  const int max_chunks = (int)std::max<long>(1, window / (4 * tile));
+  // A chunk holds at least four tiles: with fewer, the sum over a small
+  // call's chunks costs what its idle SMs would give (100x100 facets x one
+  // trace of 256 frequencies: 76 us, 99 us at one tile). Full amplitudes
+  // spend sixteen times as long on a pair and go down to one tile (32x32
+  // facets x one trace of 128 frequencies: 591 us at four, 178 us at one).
+  const long least = f64 || o->freeze_amplitudes ? 4 * tile : tile;
   const int target = 8 * sm_count();
   const int per = p->n_groups * fblk;
+  const int max_chunks = (int)std::max<long>(1, window / least);
   p->n_chunks = std::max(1, std::min(max_chunks, (target + per - 1) / per));
   p->smem = 0;
   return SS_OK;
@@ -769,7 +779,8 @@ extern "C" int ss_multifreq_response(const ss_multifreq_opts *o,
   cudaError_t e = cudaMemsetAsync(part_drop, 0, drop, st);
   if (e != cudaSuccess) return cuda_status(e, "multifreq scratch clear");
   const int fblk = (a.K + kMfFBlock - 1) / kMfFBlock;
-  const int threads = 2 * mf_half(a.K);  // split form
+  const int half = mf_half(a.K);  // split form
+  const int threads = std::max(2 * half, 32);
   dim3 grid(p.n_chunks, p.n_groups, fblk);
   if (f64) {
     if (o->freeze_amplitudes)
@@ -778,6 +789,7 @@ extern "C" int ss_multifreq_response(const ss_multifreq_opts *o,
       multifreq_fp64_kernel<true><<<grid, kMfThreads, 0, st>>>(a);
   } else {
     MfSplitConsts k{};
+    k.half = half;
     const double dfq = o->bandwidth / o->n_freq;
     const double f1 = o->f0 - 0.5 * o->bandwidth + 0.5 * dfq;
     const df rc = df_from_double(4.0 * kPi / o->c);
