@@ -235,12 +235,9 @@ int coherent_batch_fp64_launch(const BatchJob *jobs, int n_jobs,
 }
 
 int batch_fp64_blocks_per_sm(int threads, size_t smem) {
-  static size_t limit = 0;
-  limit = std::max(limit, smem);
   int n = 0;
-  if (cudaFuncSetAttribute(coherent_batch_fp64_kernel,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)limit) != cudaSuccess)
+  if (raise_smem_limit((const void *)coherent_batch_fp64_kernel, smem) !=
+      cudaSuccess)
     return 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
           &n, coherent_batch_fp64_kernel, threads, smem) != cudaSuccess)

@@ -642,15 +642,10 @@ int coherent_batch_split_launch(const BatchJob *jobs, int n_jobs,
 
 int batch_split_blocks_per_sm(int rough_kind, int form, int threads,
                               size_t smem) {
-  // raise the kernel's dynamic shared-memory limit to the largest size any
-  // prepared batch uses (never lowered: earlier batches stay launchable)
-  static size_t limit[24] = {};
-  const int r = ((rough_kind & 3) * 2 + (threads > 256 ? 1 : 0)) * 3 + form;
-  limit[r] = std::max(limit[r], smem);
+  // (several forms share a kernel: the limit goes by the kernel)
   void *fn = batch_split_fn_kind(rough_kind, threads, form);
   int n = 0;
-  cudaError_t e = cudaFuncSetAttribute(
-      fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit[r]);
+  cudaError_t e = raise_smem_limit(fn, smem);
   if (e == cudaSuccess)
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, threads, smem);
   return e == cudaSuccess ? n : 0;

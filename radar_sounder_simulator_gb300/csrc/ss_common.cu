@@ -3,7 +3,9 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <map>
 #include <mutex>
+#include <utility>
 
 #include "ss_internal.cuh"
 
@@ -22,6 +24,24 @@ int cuda_status(cudaError_t e, const char *where) {
   snprintf(buf, sizeof(buf), "%s: %s", where, cudaGetErrorString(e));
   set_error(buf);
   return SS_ERR_CUDA;
+}
+
+// Batches keep their launch parameters and may run at any time, so a kernel's
+// dynamic shared-memory limit only grows: one maximum per kernel and device,
+// whatever options led to that kernel.
+cudaError_t raise_smem_limit(const void *fn, size_t smem) {
+  static std::mutex lock;
+  static std::map<std::pair<int, const void *>, size_t> largest;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> hold(lock);
+  size_t &most = largest[{dev, fn}];
+  if (smem <= most) return cudaSuccess;
+  e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)smem);
+  if (e == cudaSuccess) most = smem;
+  return e;
 }
 
 // Weideman (1994): with M = 2N, L = sqrt(N / sqrt 2), t_k = L tan(pi k / 2M),

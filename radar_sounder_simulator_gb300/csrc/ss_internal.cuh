@@ -18,6 +18,7 @@ constexpr double kTwoPi = 6.283185307179586476925286766559005768;
 
 // Record the last CUDA error for ss_last_error().
 void set_error(const char *msg);
+cudaError_t raise_smem_limit(const void *fn, size_t smem);
 int cuda_status(cudaError_t e, const char *where);
 
 // Weideman (1994) Faddeeva constants for N = 32, computed on the host once.
