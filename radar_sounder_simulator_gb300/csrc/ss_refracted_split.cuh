@@ -1798,8 +1798,7 @@ inline int ref_batch_occupancy(int rough_kind, bool plain, size_t smem) {
   int n = 0;
   cudaError_t e = cudaSuccess;
   auto one = [&](auto kern) {
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
+    e = raise_smem_limit(reinterpret_cast<const void *>(kern), smem);
     if (e == cudaSuccess)
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern,
                                                         kSplitThreads, smem);

@@ -41,3 +41,27 @@ def test_surface_batches_of_other_forms(tuning, rough):
              batch(40, pattern=("dipole", pv, np.float64(0.), np.float64(0.)))]
     for b in first + first[::-1]:
         _same(b)
+
+
+@pytest.mark.parametrize("refraction", ["sequential", "joint"])
+@pytest.mark.parametrize("rough", [False, True])
+def test_refracted_batches_of_other_sizes(rough, refraction):
+    from radar_sounder_simulator_gb300.batch import RefractedBatch
+    from radar_sounder_simulator_gb300.multilayer import prepare_refracted
+    top, bed = _layer(20, 24, 9.0, 0.0, 1.0, 3), _layer(18, 20, 9.0, -80.0,
+                                                        1.5, 4)
+    pos, uct = _track(9, 500.0)
+    ph = np.exp(2j * np.pi * np.random.default_rng(1).random(len(bed.areas)))
+    opt = {}
+    if rough:
+        opt.update(d_phi_area=True, roughness=(
+            0.1, 2.0, ph.astype(np.complex64), 12, "exponential"))
+
+    def batch(n_samples):
+        return RefractedBatch([prepare_refracted(
+            pos, uct, bed, [top], [1.0, 3.15], [0.0, 10.0], mode="coherent",
+            refraction=refraction, k0=K0, gamma=0.2, t0=2 * 560.0 / C,
+            dt=5e-9, n_samples=n_samples, c=C, precision="split", **opt)])
+    first = [batch(1400), batch(60)]      # 87 and 4 KB of histograms
+    for b in first + first[::-1]:
+        _same(b)
