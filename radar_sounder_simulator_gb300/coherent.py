@@ -137,9 +137,11 @@ def stage_facets(centers, normals, areas, e1, e2, order, device, *,
                    device))
     soa = torch.empty((13, n), dtype=torch.float32, device=device)
     if soa.device.type == "cuda":
-        st = _lib.lib().ss_stage_facets(
-            *[t.data_ptr() for t in cols], order_t.data_ptr(), n,
-            soa.data_ptr(), torch.cuda.current_stream(soa.device).cuda_stream)
+        # a plan may be prepared for a device that is not the current one
+        with torch.cuda.device(soa.device):
+            st = _lib.lib().ss_stage_facets(
+                *[t.data_ptr() for t in cols], order_t.data_ptr(), n,
+                soa.data_ptr(), torch.cuda.current_stream().cuda_stream)
         _lib.check(st, "ss_stage_facets")
     else:
         for j, t in enumerate(cols[:4]):
