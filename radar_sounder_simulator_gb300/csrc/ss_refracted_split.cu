@@ -45,8 +45,12 @@ RefSplitConsts split_consts(const RefArgs &a) {
     double mn[3];
     for (int j = 0; j < 3; ++j) {
       mn[j] = I.mean_normal[j];
-      O.mp[j] = (float)I.mean_point[j];
-      O.mn[j] = (float)mn[j];
+      const df pd = df_from_double(I.mean_point[j]);
+      const df nd = df_from_double(mn[j]);
+      O.mp[j] = pd.hi;
+      O.mpl[j] = pd.lo;
+      O.mn[j] = nd.hi;
+      O.mnl[j] = nd.lo;
     }
     for (int c = 0; c < 4; ++c) {
       const df cd = df_from_double(I.coef[c]);
