@@ -100,17 +100,26 @@ __device__ __forceinline__ float reduce_df_2pi(float hi, float lo) {
   return __fmaf_rn(-n, -1.74845553146951e-07f, r) + lo;
 }
 
-// Sine and cosine of hi + lo (|hi| up to ~1e5) to a float32 ulp or so: the
-// argument is reduced to [-pi/4, pi/4] by quarter turns (the first product
-// exact: hi and n c share their leading bits), then the minimax polynomials
-// of Moshier's Cephes library (sinf.c) run on it, without the library
-// call's large-argument branch.
+// Sine and cosine of hi + lo, |lo| up to a few ulp of hi, by whole turns and
+// the library: the phases too large for sincos_df.
+static __device__ __noinline__ void sincos_far(float hi, float lo, float &sn,
+                                               float &cs) {
+  sincosf(reduce_df_2pi(hi, lo), &sn, &cs);
+}
+
+// Sine and cosine of hi + lo to a float32 ulp or so: the argument is reduced
+// to [-pi/4, pi/4] by quarter turns (the first product exact: hi and n c
+// share their leading bits), then the minimax polynomials of Moshier's Cephes
+// library (sinf.c) run on it, without the library call's large-argument
+// branch. The low part comes on top of the reduced angle, which the
+// polynomials bear while it is small: a float32 model gives 1.1e-7 up to 5e5
+// rad, 9e-6 at 3e6 and nonsense from 2e7 on (500 km at 1 GHz), so larger
+// phases take sincos_far.
 __device__ __forceinline__ void sincos_df(float hi, float lo, float &sn,
                                           float &cs) {
-  if (fabsf(hi) > 6e6f) {  // quarter turns beyond the integer trick: whole
-    const float m = rintf(hi * 0.159154943091895336f);  // turns first
-    hi = __fmaf_rn(-m, 6.28318548202514648f, hi);
-    lo = __fmaf_rn(m, 1.74845553146951e-07f, lo);
+  if (fabsf(hi) > 5e5f) {
+    sincos_far(hi, lo, sn, cs);
+    return;
   }
   const float t = __fmaf_rn(hi, 0.636619772367581343f, 12582912.0f);
   const int q = __float_as_int(t);

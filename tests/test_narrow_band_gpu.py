@@ -1,6 +1,7 @@
-"""Frequency synthesis of narrow bands (split form): the band response's CTA
+"""Frequency synthesis (split form) of narrow bands and of long paths. The band response's CTA
 is as wide as the band, down to two threads, so its shared tables -- four
-traces, 32 Faddeeva coefficients -- take several turns to fill. Against the
+traces, 32 Faddeeva coefficients -- take several turns to fill; a carrier phase of
+millions of radians has a low part that no longer is small. Against the
 float64 oracle within the split form's bounds (relative L2 1e-4, phase 1e-3
 rad, power 0.01 dB above -60 dB of the peak)."""
 
@@ -60,3 +61,22 @@ def test_narrow_band_matches_oracle(K, kind):
             ref.append((w / w.sum() * H) @ np.exp(
                 2j * np.pi * np.outer(freqs - kw["f0"], tw)))
     split_ok(y, np.array(ref))
+
+
+@pytest.mark.parametrize("frozen", [True, False])
+@pytest.mark.parametrize("alt,f0", [(25e3, 450e6), (400e3, 150e6),
+                                    (500e3, 1.3e9), (800e3, 5e9)])
+def test_long_paths_match_oracle(alt, f0, frozen):
+    """Carrier phases of 5e5, 2.5e6, 2.7e7 and 1.7e8 rad."""
+    from types import SimpleNamespace
+    from radar_sounder_simulator_gb300.multifreq import multifreq_traces
+    c, nr, a, e1, e2 = _scene(n=9, d=2.0, seed=4)
+    f = SimpleNamespace(centers=c, normals=nr, areas=a, e1=e1, e2=e2)
+    pos = np.column_stack([np.linspace(-80, 70, 3), np.full(3, -5.0),
+                           np.full(3, alt)])
+    tw = 2 * (alt - 8.0) / C + np.arange(24) / 30e6
+    kw = dict(gamma=-0.3, f0=f0, bandwidth=15e6, c=C, twtt=tw, n_freq=64,
+              freeze_amplitudes=frozen)
+    y = multifreq_traces(pos, c, nr, a, e1, e2, precision="split", **kw)
+    ref = np.array([omf.multifreq_profile(p, *q32(f), **kw) for p in pos])
+    split_ok(y, ref)
