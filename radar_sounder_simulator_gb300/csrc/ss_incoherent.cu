@@ -176,15 +176,16 @@ incoherent_kernel(IncArgs a) {
       const float2 S = pk(__fadd_rn(__fadd_rn(x2.x, yy.x), z2.x),
                           __fadd_rn(__fadd_rn(x2.y, yy.y), z2.y));
       const float2 y = pk(rsq_n(S.x), rsq_n(S.y));  // 1/r
-      // power (A cos)^2 / r^4 = (A (d . n))^2 / r^6
-      const float2 q =
-          mul2(ar, fma2(dz, nz, fma2(dy, ny, mul2(dx, nx))));
-      const float2 y2 = mul2(y, y);
-      float2 pw = mul2(mul2(q, q), mul2(mul2(y2, y2), y2));
       // the reference's bin coordinate
       const float2 g = mul2(S, y), hy = mul2(y, pk1(0.5f));
       const float2 r = fma2(pk(__fmaf_rn(-g.x, g.x, S.x),
                                __fmaf_rn(-g.y, g.y, S.y)), hy, g);
+      // power (A cos)^2 / r^4 = (A (d . n))^2 / r^6, 1/r to its rounding
+      const float2 q =
+          mul2(ar, fma2(dz, nz, fma2(dy, ny, mul2(dx, nx))));
+      const float2 yr = fma2(fma2(pk(-r.x, -r.y), y, pk1(1.0f)), y, y);
+      const float2 y2 = mul2(yr, yr);
+      float2 pw = mul2(mul2(q, q), mul2(mul2(y2, y2), y2));
       const float ex = __fmaf_rn(-r.x, r.x, S.x),
                   ey = __fmaf_rn(-r.y, r.y, S.y);
       // 2^k of the binade just below r: a power of two's lower neighbour is
