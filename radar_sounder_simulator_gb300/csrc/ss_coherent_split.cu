@@ -38,16 +38,17 @@
 // Everything else (incidence, sincs, taper, antenna gain, roughness series)
 // runs in float32 from q + w and the facet's per-block products;
 // histograms accumulate float32 per CTA chunk and the reduce kernel sums
-// the chunks by float32 two-sums (~2^-48 relative). A bin is one 8-byte
-// (re, im) cell updated by a 64-bit compare-and-swap (hist_add): one shared
-// round trip per pair where two float atomics -- loops of 32-bit
-// compare-and-swaps in shared memory -- took two.
+// the chunks by float32 two-sums (~2^-48 relative). A bin is an (re, im) cell
+// of two float32 atomics, each a loop of 32-bit compare-and-swaps in shared
+// memory. One 64-bit compare-and-swap for both saves a round trip where lanes
+// rarely meet (512^2 facets x 1024 traces 2.58 ms of the sum and its SAR
+// image, 2.67 with two), but its retries cost far more where they do: 24x21
+// facets x 71 traces 61 us against 30, 10x165 x 78 into 64 bins 517 against
+// 114, a sweep of six surfaces 1.11 ms against 1.05.
 //
-// Bound by instruction issue, ~240 instructions per pair (307 with a
-// division for dr, two atomics and denormal handling in the special
-// functions): 512^2 facets x 1024 traces with an antenna pattern 2.45 ->
-// 1.85 ms; 128^2 x 256, which is half set-up and reduce, 133 -> 104 us with
-// both.
+// Bound by instruction issue, ~260 instructions per pair (307 with a
+// division for dr and denormal handling in the special functions): 128^2 x
+// 256, which is half set-up and reduce, 133 -> 105 us.
 #include <algorithm>
 
 #include "ss_coherent.cuh"
@@ -491,13 +492,17 @@ __device__ __forceinline__ void coherent_split_cta(const CoArgs &a,
           const float bq = fb + (float)q;
           const float pr = re * wq[q], pim = im * wq[q];
           if (bq >= 0.0f && bq < nsf) {
-            hist_add(hist + row + small_int(bq), pr, pim);
+            float2 *h = hist + row + small_int(bq);
+            atomicAdd(&h->x, pr);
+            atomicAdd(&h->y, pim);
           } else {
             drop += pr * pr + pim * pim;
           }
         }
       } else if (fb >= 0.0f && fb < nsf) {
-        hist_add(hist + row + small_int(fb), re, im);
+        float2 *h = hist + row + small_int(fb);
+        atomicAdd(&h->x, re);
+        atomicAdd(&h->y, im);
       } else {
         drop = re * re + im * im;
       }

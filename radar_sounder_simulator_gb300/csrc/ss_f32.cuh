@@ -85,23 +85,6 @@ __device__ __forceinline__ float sinc_n(float x) {
   return sin_n(reduce_2pi(x)) * rcp_n(x);
 }
 
-// (re, im) into a bin of a shared-memory histogram by one 64-bit
-// compare-and-swap: two float atomics are two such loops of 32 bits.
-__device__ __forceinline__ void hist_add(float2 *h, float re, float im) {
-  unsigned long long *p = reinterpret_cast<unsigned long long *>(h);
-  unsigned long long old = *reinterpret_cast<volatile unsigned long long *>(p),
-                     was;
-  do {
-    was = old;
-    const float2 v =
-        make_float2(__int_as_float((int)was) + re,
-                    __int_as_float((int)(was >> 32)) + im);
-    old = atomicCAS(p, was,
-                    ((unsigned long long)(unsigned)__float_as_int(v.y) << 32) |
-                        (unsigned)__float_as_int(v.x));
-  } while (old != was);
-}
-
 __device__ __forceinline__ float dot3f(float ax, float ay, float az, float bx,
                                        float by, float bz) {
   return __fmaf_rn(az, bz, __fmaf_rn(ay, by, ax * bx));

@@ -1415,13 +1415,8 @@ __device__ __forceinline__ void refracted_split_cta(const RefArgs &a,
       }
       if (o.bin >= 0) {
         float2 *h = hist + (size_t)tt * a.n_seg + o.bin;
-        if (NI < 0) {
-          hist_add(h, o.re, o.im);
-        } else {
-          // (the general form's 64 registers are full: one value at a time)
-          atomicAdd(&h->x, o.re);
-          if (a.coherent) atomicAdd(&h->y, o.im);
-        }
+        atomicAdd(&h->x, o.re);
+        if (a.coherent) atomicAdd(&h->y, o.im);
       } else {
         atomicAdd(&s_drop[tt], o.pwr);
       }
