@@ -351,6 +351,12 @@ static __device__ __noinline__ bool joint_solve64(
   for (int it = 0; it < n_newton && !done; ++it) {
     F delta[NI][2];
     const F dmax = joint_step<NI, F>(G, BB, nm, delta, ni);
+    // A step below 1e-9 of the shortest leg is rounding, and leaves 1e-18 of
+    // it. (Of the path it would leave a metre-long leg under 20 km with a
+    // residual past the validity limit.)
+    double shortest = G.s[0];
+    for (int i = 1; i <= ni; ++i) shortest = fmin(shortest, G.s[i]);
+    const bool last = dmax < (F)1e-9 * (F)fmin(shortest, 1.0);
     // step halving on |F|^2; the accepted candidate's geometry is the next
     // iteration's
     const double m0 = G.m;
@@ -364,9 +370,9 @@ static __device__ __noinline__ bool joint_solve64(
         for (int r = 0; r < 2; ++r)
           ab[i][r] = keep[i][r] + lam * (double)delta[i][r];
       joint_geom<NI>(B, D, nm, ab, G, ni);
-      // below 1e-9 of the path scale the residual is rounding: the step
-      // itself is the correction
-      if (G.m < m0 || (dmax < (F)1e-9 && isfinite(G.m))) {
+      // in a last step the residual is rounding: the step itself is the
+      // correction
+      if (G.m < m0 || (last && isfinite(G.m))) {
         moved = true;
         break;
       }
@@ -377,7 +383,7 @@ static __device__ __noinline__ bool joint_solve64(
       joint_geom<NI>(B, D, nm, ab, G, ni);
       break;
     }
-    done = dmax < (F)1e-9;  // the remaining error is below rounding
+    done = last;
   }
   // crossings, legs and validity (refraction_joint.py:143-176): with
   // orthonormal bases the in-plane parts are the projections
