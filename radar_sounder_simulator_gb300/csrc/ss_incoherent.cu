@@ -37,7 +37,7 @@
 //
 // Bound by instruction issue (63 per pair, 68% of the slots at 32 warps per
 // SM, a third of them the histogram's compare-and-swap loops): 512^2 facets x
-// 1024 traces 855 -> 640 us.
+// 1024 traces 855 -> 652 us.
 #include <algorithm>
 #include <cstdint>
 #include <cstring>
@@ -79,16 +79,15 @@ __device__ __forceinline__ float2 div_const2(float2 x, float z, float zl,
   return fma2(fma2(q, pk1(nb), x), pk1(z), q);
 }
 
-// CTA size: two 512-thread CTAs (64 registers) hold 32 warps per SM where
-// 256-thread ones (73 registers, and room for three 64 KB histograms) hold
-// 24; an antenna pattern needs twice the registers.
-template <bool PAT>
-constexpr int inc_threads() {
-  return PAT ? 256 : 512;
-}
+// Two 512-thread CTAs (64 registers) hold 32 warps per SM, with or without an
+// antenna pattern: a pattern's 136 registers in 256-thread CTAs left eight
+// (512^2 facets x 1024 traces with a dipole 2.49 -> 1.16 ms, with a table
+// 4.16 -> 1.88 ms; three or four 256-thread CTAs per SM 1.25 and 1.31, 1.98
+// and 2.14).
+constexpr int kIncThreads = 512;
 
 template <int TB, bool PAT>
-__global__ void __launch_bounds__(inc_threads<PAT>(), PAT ? 1 : 2)
+__global__ void __launch_bounds__(kIncThreads, 2)
 incoherent_kernel(IncArgs a) {
   extern __shared__ __align__(16) float hist[];  // (TB, stride)
   __shared__ float4 s_p[TB], s_u[TB];
@@ -328,7 +327,7 @@ int inc_launch_t(const IncArgs &a, const IncPlan &p, cudaStream_t st) {
       (int)p.smem);
   if (e != cudaSuccess) return cuda_status(e, "incoherent smem");
   dim3 grid(p.n_chunks, p.n_groups);
-  incoherent_kernel<TB, PAT><<<grid, inc_threads<PAT>(), p.smem, st>>>(a);
+  incoherent_kernel<TB, PAT><<<grid, kIncThreads, p.smem, st>>>(a);
   return cuda_status(cudaGetLastError(), "incoherent launch");
 }
 
