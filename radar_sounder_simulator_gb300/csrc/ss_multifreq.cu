@@ -789,7 +789,14 @@ extern "C" int ss_multifreq_response(const ss_multifreq_opts *o,
   if (e != cudaSuccess) return cuda_status(e, "multifreq scratch clear");
   const int fblk = (a.K + kMfFBlock - 1) / kMfFBlock;
   const int half = mf_half(a.K);  // split form
-  const int threads = std::max(2 * half, 32);
+  // a rough pair's series wants more of the tile's pairs done at once: all of
+  // them with the Faddeeva terms (32x32 facets x 5 traces of 455 frequencies,
+  // 60 terms: 225 us, 365 with 64 threads), two turns without (100x100 x 100
+  // of 300: 277 us, 322 with 128)
+  const int threads =
+      rk == SS_ROUGH_GAUSS_FULL
+          ? kMfThreads
+          : std::max(2 * half, rk != SS_ROUGH_NONE ? 64 : 32);
   dim3 grid(p.n_chunks, p.n_groups, fblk);
   if (f64) {
     if (o->freeze_amplitudes)
