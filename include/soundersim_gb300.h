@@ -443,9 +443,11 @@ typedef struct {
   int32_t ctas_per_sm;   /* persistent CTAs per SM (default: as many as fit) */
 } ss_batch_tuning;
 
-/* Filled by ss_coherent_batch_prepare; passed back to ss_coherent_batch_run. */
+/* Filled by ss_coherent_batch_prepare; passed back, unchanged, to
+ * ss_coherent_batch_run. form: the kernel form every job fits (0 any options,
+ * 1 an antenna pattern at most, 2 none). */
 typedef struct {
-  int32_t n_jobs, precision, rough_kind, threads, ctas, reserved;
+  int32_t n_jobs, precision, rough_kind, threads, ctas, form;
   int64_t n_items, n_out;
   uint64_t smem, table_offset;
 } ss_batch_info;
@@ -483,8 +485,10 @@ typedef struct {
   ss_output out;
 } ss_refracted_job;
 
-/* Filled by ss_refracted_batch_prepare; passed back to
- * ss_refracted_batch_run. */
+/* Filled by ss_refracted_batch_prepare; passed back, unchanged, to
+ * ss_refracted_batch_run. plain: bit 0 when no job has an option (roughness,
+ * pattern, taper, diffuse channel, side split), bit 1 when every job takes
+ * the short form of the batch's path class. */
 typedef struct {
   int32_t n_jobs, path_class, rough_kind, plain, ctas, reserved;
   int64_t n_items, n_out, n_words;

@@ -186,7 +186,7 @@ class RefractedBatchInfo(C.Structure):
 class BatchInfo(C.Structure):
     _fields_ = [("n_jobs", C.c_int32), ("precision", C.c_int32),
                 ("rough_kind", C.c_int32), ("threads", C.c_int32),
-                ("ctas", C.c_int32), ("reserved", C.c_int32),
+                ("ctas", C.c_int32), ("form", C.c_int32),
                 ("n_items", C.c_int64), ("n_out", C.c_int64),
                 ("smem", C.c_uint64), ("table_offset", C.c_uint64)]
 

@@ -93,8 +93,8 @@ class CoherentBatch:
                     for p in self.plans)
         nseg = max(p.n_seg for p in self.plans)
         return (len(self.plans), self.precision,
-                int(self.plans[0].rst.kind), int(round(math.log2(
-                    max(pairs, 1)))), nseg,
+                int(self.plans[0].rst.kind), self.info.form,
+                int(round(math.log2(max(pairs, 1)))), nseg,
                 torch.cuda.get_device_name(self.device))
 
     def prepare(self, tuning):

@@ -208,7 +208,7 @@ extern "C" int ss_coherent_batch_prepare(const ss_coherent_job *jobs,
   info->precision = L.precision;
   info->rough_kind = L.rough_kind;
   info->threads = L.threads;
-  info->reserved = L.form;  // the kernel form every job fits
+  info->form = L.form;  // the kernel form every job fits
   info->ctas = per_sm * sm_count();
   info->n_items = L.n_items;
   info->n_out = L.n_out;
@@ -237,7 +237,7 @@ extern "C" int ss_coherent_batch_run(const ss_batch_info *info,
                                            info->smem, st)
               : coherent_batch_split_launch(jobs, info->n_jobs,
                                             info->n_items, counter,
-                                            info->rough_kind, info->reserved,
+                                            info->rough_kind, info->form,
                                             info->threads, info->ctas,
                                             info->smem, st);
   if (s) return s;
