@@ -104,9 +104,10 @@ __device__ __forceinline__ void coherent_fp64_cta(const CoArgs &a, int chunk,
       const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx),
                                             __dmul_rn(dy, dy)),
                                   __dmul_rn(dz, dz));
-      const double ir = rsqrt(r2);
+      double ir = rsqrt(r2);
       double r = r2 * ir;
       r = fma(fma(-r, r, r2), 0.5 * ir, r);
+      ir = fma(fma(-r, ir, 1.0), ir, ir);  // 1/r to its rounding
       const double cosv = dot3(dx, dy, dz, nx, ny, nz) * ir;
       const double d1 = dot3(dx, dy, dz, e1x, e1y, e1z) * ir;
       const double d2 = dot3(dx, dy, dz, e2x, e2y, e2z) * ir;
