@@ -21,10 +21,9 @@
 //     in float32). N is thus a double-float; dr is the float32 difference
 //     of the two ranges (right to an ulp of the range) and one Newton step
 //     of that equation, whose residual is formed exactly and whose slope is
-//     2 r_t: no division, and dr good to ~2e-11 of its size (3e-9 m at
-//     |w| = 160 m; a float32 dr would carry ulp(|w|)/2 of rounding: 4e-6 m
-//     at 100 m, 8e-5 rad of phase at 450 MHz). The middle trace has w = 0
-//     and its pairs are exact to the reference's double-float.
+//     2 r_t: no division, and dr good to ~1.4e-9 m at 20 km, the middle
+//     trace (w = 0) included (a float32 dr would carry ulp(|w|)/2 of
+//     rounding: 4e-6 m at 100 m, 8e-5 rad of phase at 450 MHz).
 //
 // The bin position ubc + fc + A dr is then good to ~2e-7 bins; a pair
 // within 2e-6 bins of an edge recomputes its own double-float range and
@@ -402,7 +401,7 @@ __device__ __forceinline__ void coherent_split_cta(const CoArgs &a,
       const float Nl = g + lw.z;
       // float32 r_t; dr = r_t - r_c to its rounding, then one Newton step of
       // dr^2 + 2 r_c dr = N from the exact residual: the step carries the
-      // low part (up to an ulp of r), and dr is good to ~1e-10 m
+      // low part (up to an ulp of r), and dr is good to ~1.4e-9 m at 20 km
       const float rr = __fmaf_rn(rch, rch, Nh);
       const float inv_r = rsq_n(rr);
       const float dr = __fmaf_rn(rr, inv_r, -rch);

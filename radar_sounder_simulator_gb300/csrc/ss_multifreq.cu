@@ -23,8 +23,8 @@
 //   binned split kernel); FP64 form: float64 throughout.
 // Synthesis (T x K x B): thread <-> output sample; the factor
 //   exp(2j pi (f_k - f0) twtt_b) is re-anchored every 8 frequencies from a
-//   float64 cycle count and rotated in between; split-form sums are
-//   compensated (two-sum).
+//   cycle count (double-float in the split form, two samples per thread) and
+//   rotated in between; split-form sums are compensated (two-sum).
 #include <algorithm>
 
 #include "ss_df.cuh"

@@ -278,7 +278,11 @@ static int refracted_plan(const ss_refracted_opts *o, int T, int N, Plan *p) {
   } else {
     // resident CTAs per SM of the split kernel that runs: two 512-thread
     // CTAs (64 registers) for the sequential chain and joint solves through
-    // one interface, one (~128 registers) through two or more
+    // one interface, one (~128 registers) for the lean form through two and
+    // either form through more. (The general form through two runs two as
+    // well but is planned as one: 180x200 facets x 200 traces with rough
+    // crossings 0.95 ms, 1.07 planned as two; 90x300 x 97 0.50, 0.55; alike
+    // from 256^2 x 300 on.)
     const int max_chunks = (int)std::max<long>(1, window / 256);
     const long slots = (long)sm_count() *
                        (!o->joint || o->n_crossed <= 1 ? 2 : 1);

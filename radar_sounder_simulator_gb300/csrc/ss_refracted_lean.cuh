@@ -19,7 +19,7 @@
 //   * The residual, the legs' lengths and the heights off the planes are as
 //     in the general form; transmission takes both Snell cosines.
 //
-// 512^2 facets x 1024 traces through three interfaces: 43.8 -> 19.9 ms (2,060
+// 512^2 facets x 1024 traces through three interfaces: 43.8 -> 20.6 ms (2,060
 // instructions per pair; issue 77% at 16 warps per SM, FMA pipe 60%).
 #pragma once
 

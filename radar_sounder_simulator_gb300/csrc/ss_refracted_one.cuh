@@ -24,7 +24,7 @@
 //     1 - gamma^2 = 4 n1 c1 n2 c2 / (n1 c1 + n2 c2)^2, and the spreading and
 //     flux factors folded into one quotient.
 //
-// 512^2 facets x 1024 traces under one interface: 12.4 -> 5.2 ms (1,542 ->
+// 512^2 facets x 1024 traces under one interface: 12.4 -> 5.3 ms (1,542 ->
 // 640 instructions per pair; issue 88%, FMA pipe 60%).
 #pragma once
 

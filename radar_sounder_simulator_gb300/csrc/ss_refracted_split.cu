@@ -142,7 +142,7 @@ bool one_crossing(const RefArgs &a) {
 
 bool lean_joint(const RefArgs &a) {
   // Up to kLeanMax interfaces the lean form takes half the general form's time
-  // (three: 43.8 and 19.9 ms for 512^2 facets x 1024 traces); deeper stacks
+  // (three: 43.8 and 20.6 ms for 512^2 facets x 1024 traces); deeper stacks
   // keep the arrays of the general form. A histogram beyond the usual budget
   // leaves no room for the constants.
   return (size_t)a.n_seg * sizeof(float2) <= 96 * 1024 && a.joint &&

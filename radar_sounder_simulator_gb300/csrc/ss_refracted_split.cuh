@@ -21,7 +21,10 @@
 //     to ~5e-5 cells of float32 error through three interfaces); within
 //     1.5e-4 cells of a rounding boundary the float64 mean-plane chain of
 //     the reference is re-run for that pair, so the lookups are the
-//     reference's integer decisions;
+//     reference's integer decisions. (Flat rays, beyond 49 degrees on the
+//     rarer side, are the exception: the reference's ten iterations may stop
+//     short of the root, which the short paths' lookups always reach; a pair
+//     deferred to the fix-up takes the ten iterations);
 //   * leg lengths, optical path, carrier phase (2 k0 opl mod 2 pi) and the
 //     fast-time bin in double-float. The optical path is stationary in the
 //     crossing positions along the interface (Fermat), so that float32
